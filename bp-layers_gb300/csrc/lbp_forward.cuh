@@ -90,22 +90,17 @@ struct FwdArgs {
 // ((float)exp((double)m) and (float)log(max((double)sum, 1e-45)),
 // lbp_min_sum_kernel.cu:167, :180-181): correctly rounded float-float
 // evaluation, double precision only when the rounding is undecided.
-__device__ __forceinline__ float norm_exp(float m, const float* ehi, const float* elo) {
-  float y;
-  if (!crm::exp_fast(m, y, ehi, elo)) y = static_cast<float>(exp(static_cast<double>(m)));
-  return y;
-}
 // exp of the normalisation: the exact evaluation above (float storage) or
 // the hardware approximation (half storage, not bit-exact by design)
 template <bool EXACT>
-__device__ __forceinline__ bool exp_try(float x, float& y, const float* ehi, const float* elo) {
-  if (EXACT) return crm::exp_fast(x, y, ehi, elo);
+__device__ __forceinline__ bool exp_try(float x, float& y, const crm::ExpEntry* tab) {
+  if (EXACT) return crm::exp_fast(x, y, tab);
   y = __expf(x);
   return true;
 }
-__device__ __forceinline__ float norm_log(float sum) {
+__device__ __forceinline__ float norm_log(float sum, const crm::LogEntry* tab) {
   float y;
-  if (!crm::log_fast(sum, y)) y = static_cast<float>(log(fmax(static_cast<double>(sum), 1e-45)));
+  if (!crm::log_fast(sum, y, tab)) y = static_cast<float>(log(fmax(static_cast<double>(sum), 1e-45)));
   return y;
 }
 
@@ -396,12 +391,15 @@ __global__ void __launch_bounds__(32 * fwd_block_warps<OCC>(), OCC) lbp_forward_
     p += 2 * align4(a.ns);
     sm.taps = p;
   }
-  // exp table for lane-varying lookups: every warp writes the same values
-  __shared__ float s_ehi[64], s_elo[64];
-  s_ehi[lane] = crm::kTab.exp_hi[lane];
-  s_ehi[lane + 32] = crm::kTab.exp_hi[lane + 32];
-  s_elo[lane] = crm::kTab.exp_lo[lane];
-  s_elo[lane + 32] = crm::kTab.exp_lo[lane + 32];
+  // exp and log tables: every warp writes the same values
+  __shared__ crm::ExpEntry s_exp[kExact ? crm::kExpEntries : 1];
+  __shared__ crm::LogEntry s_log[kExact ? crm::kLogEntries : 1];
+  if constexpr (kExact) {
+#pragma unroll
+    for (int q = 0; q < crm::kExpEntries / 32; ++q) s_exp[lane + 32 * q] = crm::kTab.e[lane + 32 * q];
+#pragma unroll
+    for (int q = 0; q < crm::kLogEntries / 32; ++q) s_log[lane + 32 * q] = crm::kTab.l[lane + 32 * q];
+  }
   if (wic == 0 && lane < kHsPad) {
     cs.hs[-1 - lane] = __int_as_float(0x7f800000);
     cs.hs[32 * K + lane] = __int_as_float(0x7f800000);
@@ -678,7 +676,7 @@ __global__ void __launch_bounds__(32 * fwd_block_warps<OCC>(), OCC) lbp_forward_
       }
       msg[0] = (lane < L) ? m : 1e15f;
       am[0] = (lane < L) ? arg : 0;
-      bool eok0 = exp_try<kExact>(earg(msg[0]), e[0], s_ehi, s_elo);
+      bool eok0 = exp_try<kExact>(earg(msg[0]), e[0], s_exp);
       if (lane >= L) {
         e[0] = 0.0f;
         eok0 = true;
@@ -714,7 +712,7 @@ __global__ void __launch_bounds__(32 * fwd_block_warps<OCC>(), OCC) lbp_forward_
       bool eok[KW];
 #pragma unroll
       for (int kk = 0; kk < KW; ++kk) {
-        eok[kk] = exp_try<kExact>(earg(msg[kk]), e[kk], s_ehi, s_elo);
+        eok[kk] = exp_try<kExact>(earg(msg[kk]), e[kk], s_exp);
         if (c.t0 + lane + 32 * kk >= L) {
           e[kk] = 0.0f;
           eok[kk] = true;
@@ -989,7 +987,7 @@ __global__ void __launch_bounds__(32 * fwd_block_warps<OCC>(), OCC) lbp_forward_
       }
       if (nslot <= 1 && bsel != FULL) {
         float y;
-        const bool okx = exp_try<kExact>(earg(xs), y, s_ehi, s_elo);
+        const bool okx = exp_try<kExact>(earg(xs), y, s_exp);
         all_ok = __all_sync(FULL, okx);
         e_g = __shfl_sync(FULL, y, __ffs(~bsel) - 1);
 #pragma unroll
@@ -1013,7 +1011,7 @@ __global__ void __launch_bounds__(32 * fwd_block_warps<OCC>(), OCC) lbp_forward_
         if (n_own < 32) {
           const float x = (lane < n_own) ? eb[lane] : msg_g;
           float y;
-          const bool okx = exp_try<kExact>(earg(x), y, s_ehi, s_elo);
+          const bool okx = exp_try<kExact>(earg(x), y, s_exp);
           all_ok = __all_sync(FULL, lane > n_own || okx);
           __syncwarp();
           if (lane < n_own) eb[lane] = y;
@@ -1027,14 +1025,14 @@ __global__ void __launch_bounds__(32 * fwd_block_warps<OCC>(), OCC) lbp_forward_
           }
         } else {
           // more than a warp's worth: one pass per slot that has own labels
-          all_ok = exp_try<kExact>(earg(msg_g), e_g, s_ehi, s_elo);
+          all_ok = exp_try<kExact>(earg(msg_g), e_g, s_exp);
 #pragma unroll
           for (int kk = 0; kk < KW; ++kk) {
             const bool valid = lvalid(kk);
             e[kk] = valid ? e_g : 0.0f;
             if (__any_sync(FULL, own[kk])) {
               float ex;
-              const bool okx = exp_try<kExact>(earg(msg[kk]), ex, s_ehi, s_elo);
+              const bool okx = exp_try<kExact>(earg(msg[kk]), ex, s_exp);
               e[kk] = own[kk] ? ex : e[kk];
               all_ok = all_ok && (okx || !own[kk]);
             }
@@ -1067,7 +1065,7 @@ __global__ void __launch_bounds__(32 * fwd_block_warps<OCC>(), OCC) lbp_forward_
       float ev[K];
 #pragma unroll
       for (int k = 0; k < K; ++k) ev[k] = e[k % KW];
-      sum = tree_sum<K>(ev, L, lane);
+      sum = tree_sum<K>(ev);
     } else {
 #pragma unroll
       for (int kk = 0; kk < KW; ++kk) cs.erow[c.t0 + lane + 32 * kk] = e[kk];
@@ -1075,11 +1073,11 @@ __global__ void __launch_bounds__(32 * fwd_block_warps<OCC>(), OCC) lbp_forward_
       float ev[K];
 #pragma unroll
       for (int k = 0; k < K; ++k) ev[k] = cs.erow[lane + 32 * k];
-      sum = tree_sum<K>(ev, L, lane);
+      sum = tree_sum<K>(ev);
     }
     // subtracted from every label: log of the sum (the reference's
     // normalisation) for float storage, the minimum of h for half storage
-    const float lse = kExact ? norm_log(sum) : ref;
+    const float lse = kExact ? norm_log(sum, s_log) : ref;
 
     // write the message at the receiver
     const int pq = pin + c.dpin;
@@ -1149,7 +1147,8 @@ int launch_phase(const FwdArgs& a0, cudaStream_t stream) {
     for (int ns = a.ns; ns >= 2; --ns) {
       const size_t pc = 4 * (static_cast<size_t>(chain_smem_floats(K)) +
                              static_cast<size_t>(warp_smem_floats(ns, lroww, a.lmat, a.Lv, sizeof(T))));
-      const int per_sm = std::min(32, static_cast<int>(smem_per_sm() / (pc + smem_reserved_per_block())));
+      const size_t tabs = (sizeof(T) == 4) ? sizeof(crm::Tables) : 0;
+      const int per_sm = std::min(32, static_cast<int>(smem_per_sm() / (pc + tabs + smem_reserved_per_block())));
       a.ns = ns;
       if (static_cast<int64_t>(per_sm) * sm_count() >= a.nchains) break;
     }
