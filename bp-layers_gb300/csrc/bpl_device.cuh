@@ -118,6 +118,21 @@ __device__ __forceinline__ float ord2f(unsigned u) {
 }
 __device__ __forceinline__ float warp_min_redux(float v) { return ord2f(__reduce_min_sync(0xffffffffu, f2ord(v))); }
 
+// The warp minimum by the float form of redux.sync: no key conversion before
+// and after it.  NaNs are ignored unless every lane holds one.
+__device__ __forceinline__ float warp_min_f32(float v) {
+  float r;
+  asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
+}
+
+// min(a, b, c) in one instruction (a NaN operand is ignored, like fminf).
+__device__ __forceinline__ float fmin3(float a, float b, float c) {
+  float r;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+
 // Reduce-scatter of 8 per-lane values over the warp in 9 shuffles (instead
 // of 8 full warp sums): returns in every lane the warp total of value
 // (lane >> 2) & 7, i.e. lanes 4b..4b+3 hold the total of value b.  Any
@@ -239,6 +254,8 @@ template <int N>
 __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
+
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
 // float -> unsigned short as the reference's static_cast compiles (PTX
 // float-to-integer conversions clamp to the destination range, NaN -> 0).

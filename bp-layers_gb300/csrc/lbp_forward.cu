@@ -53,6 +53,9 @@ int lbp_forward_impl(int storage, int variant, const void* cost, const void* jum
   a.eb = edge_batch;
   a.delta = delta;
   a.argmin_kind = argmin_kind;
+  a.am_vec = (reinterpret_cast<uintptr_t>(argmin) | static_cast<uintptr_t>(L)) % 16 == 0  ? 16
+             : (reinterpret_cast<uintptr_t>(argmin) | static_cast<uintptr_t>(L)) % 4 == 0 ? 4
+                                                                                          : 1;
   a.planes2 = planes2;
   a.lrow = align4(L);
   if (storage == 0) {

@@ -21,6 +21,15 @@
 //     them instead through a per-warp shared-memory ring NS pixels ahead with
 //     TMA 1-D bulk copies (cp.async.bulk + mbarrier, bounded waits), or
 //     4-byte cp.async when a row is not 16-byte sized.
+//   * The stereo float step has a hot loop for the usual window (store_lean):
+//     one straight-line block with one vote, instead of branches per case and
+//     label group.  What bounds it: along rows the latency of one step
+//     (376x1240x192: 752 warps on 608 SM sub-partitions; about 430
+//     instructions and 1300 cycles a step where the general step takes 770
+//     and 2900), down columns DRAM (1.1 GB read per direction and 0.45
+//     written, 80 % of the copy rate).  A forward pass at 376x1240x192 went
+//     from 2.48 to 1.38 ms (rows 1.50 -> 0.83, columns 0.98 -> 0.55), at
+//     188x620x96 from 0.82 to 0.42 ms, at 4x256x512x96 from 1.34 to 0.79 ms.
 //   * Labels are spread over lanes (label = lane + 32k).  min/argmin and the
 //     exp-sum reproduce the reference's reduction tree (bpl_device.cuh); the
 //     exp/log of the normalisation are correctly rounded float evaluations
@@ -31,6 +40,7 @@
 #include <cuda_fp16.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "bpl_crmath.cuh"
 #include "bpl_device.cuh"
@@ -54,6 +64,8 @@ constexpr int kHsPad = 4;
 // scanline's labels over several warps (0: never; the split pays only when
 // the per-label work dominates the per-step reductions).
 constexpr int kSplitChainsPerSm = 0;
+// steps ahead of the L2 prefetch of a lean launch with few warps per SM
+constexpr int kL2Ahead = 3;
 // scanlines per SM above which a phase runs the high-occupancy instantiation
 constexpr int kHiOccChainsPerSm = 8;
 
@@ -72,6 +84,7 @@ struct FwdArgs {
   int Ls;     // label stride of cost / messages / argmin rows
   int Lm;     // row stride of the pixel-pairwise matrices (pixel variant)
   int argmin_kind;
+  int am_vec;  // uint8 argmin rows start on multiples of this many bytes and are multiples of it long (16, 4 or 1)
   int phase;  // 0: RIGHT+LEFT over rows, 1: DOWN+UP over columns
   int nchains;
   int ns;     // ring depth (steps)
@@ -127,8 +140,17 @@ __host__ __device__ inline int ring_floats(int ns, int lroww, int lmat, int tsiz
   return align4((ns * stage_elems(lroww, lmat) * tsize + 3) / 4);
 }
 
-__host__ __device__ inline int warp_smem_floats(int ns, int lroww, int lmat, int Lv, int tsize) {
-  return ring_floats(ns, lroww, lmat, tsize) + 2 * align4(ns) + align4(2 * tap_tile_rows(Lv) * 33);
+// Lean records of a tap tile (stereo, float storage): per sender the float4
+// {w, L2, f(t-1), f(t+1)} and the float2 {f(t-2), f(t+2)}, see store_lean.
+constexpr int kLeanFloats = 32 * 6;
+// offset of the lean records within a tap tile, and the tile's length
+__host__ __device__ inline int lean_off(int Lv) { return align4(tap_tile_rows(Lv) * 33); }
+__host__ __device__ inline int tap_tile_floats(int Lv, bool lean) {
+  return lean ? lean_off(Lv) + kLeanFloats : tap_tile_rows(Lv) * 33;
+}
+
+__host__ __device__ inline int warp_smem_floats(int ns, int lroww, int lmat, int Lv, int tsize, bool lean) {
+  return ring_floats(ns, lroww, lmat, tsize) + 2 * align4(ns) + align4(2 * tap_tile_floats(Lv, lean));
 }
 
 template <typename T>
@@ -281,6 +303,41 @@ constexpr int kWinGeneric = 0;
 constexpr int kWinHasTieOnly = 0x100;
 constexpr int kWinTieIsL2 = 0x200;  // every tie-only tap equals L2 bitwise
 
+// Classifies the tile column of this lane's sender (its taps and edge weight
+// are in the tile; no other lane's values are read).
+__device__ __forceinline__ void classify_taps(const FwdArgs& a, float* tile, int lane) {
+  const float w = tile[a.Lv * 33 + lane];
+  const float L2 = tile[(a.Lv - 1) * 33 + lane];
+  int code = kWinGeneric;
+  float fnr = 0.0f;
+  if (tile[lane] == 0.0f && a.delta <= kFastDelta) {
+    int R = -1;
+    bool ok = true, seen_tie = false, have_tie = false, tie_l2 = true;
+    for (int q = 0; q <= a.delta; ++q) {
+      const float fp = tile[max(1, min(a.Lv - 1, a.Lv / 2 - q)) * 33 + lane];  // jd = +q
+      const float fm = tile[max(1, min(a.Lv - 1, a.Lv / 2 + q)) * 33 + lane];  // jd = -q
+      const bool tp = (w > 0.0f) ? (fp >= L2) : ((w < 0.0f) ? (fp <= L2) : true);
+      const bool tm = (w > 0.0f) ? (fm >= L2) : ((w < 0.0f) ? (fm <= L2) : true);
+      if (!tp && !tm) {
+        if (seen_tie) ok = false;
+        R = q;
+      } else if (tp && tm) {
+        seen_tie = true;
+        tie_l2 = tie_l2 && __float_as_int(fp) == __float_as_int(L2) && __float_as_int(fm) == __float_as_int(L2);
+        // tie-only tap of smallest product f*w
+        const float f = (w >= 0.0f) ? fminf(fp, fm) : fmaxf(fp, fm);
+        fnr = !have_tie ? f : ((w >= 0.0f) ? fminf(fnr, f) : fmaxf(fnr, f));
+        have_tie = true;
+      } else {
+        ok = false;
+      }
+    }
+    if (ok && R <= 2) code = (R + 2) | (have_tie ? kWinHasTieOnly : 0) | ((have_tie && tie_l2) ? kWinTieIsL2 : 0);
+  }
+  tile[(a.Lv + 1) * 33 + lane] = fnr;
+  tile[(a.Lv + 2) * 33 + lane] = __int_as_float(code);
+  }
+
 __device__ __forceinline__ void store_taps(const FwdArgs& a, float* tile, int lane, const TapRegs& r,
                                            bool stereo) {
   // tile layout: [Lv+3][33]; rows 0..Lv-1 taps, row Lv the edge weight,
@@ -290,38 +347,66 @@ __device__ __forceinline__ void store_taps(const FwdArgs& a, float* tile, int la
 #pragma unroll
     for (int k = 0; k < 16; ++k)
       if (k < a.Lv) tile[k * 33 + lane] = r.t[k];
-    // each lane classifies its own column (no other lane's values are read)
-    const float w = r.w;
-    const float L2 = tile[(a.Lv - 1) * 33 + lane];
-    int code = kWinGeneric;
-    float fnr = 0.0f;
-    if (tile[lane] == 0.0f && a.delta <= kFastDelta) {
-      int R = -1;
-      bool ok = true, seen_tie = false, have_tie = false, tie_l2 = true;
-      for (int q = 0; q <= a.delta; ++q) {
-        const float fp = tile[max(1, min(a.Lv - 1, a.Lv / 2 - q)) * 33 + lane];  // jd = +q
-        const float fm = tile[max(1, min(a.Lv - 1, a.Lv / 2 + q)) * 33 + lane];  // jd = -q
-        const bool tp = (w > 0.0f) ? (fp >= L2) : ((w < 0.0f) ? (fp <= L2) : true);
-        const bool tm = (w > 0.0f) ? (fm >= L2) : ((w < 0.0f) ? (fm <= L2) : true);
-        if (!tp && !tm) {
-          if (seen_tie) ok = false;
-          R = q;
-        } else if (tp && tm) {
-          seen_tie = true;
-          tie_l2 = tie_l2 && __float_as_int(fp) == __float_as_int(L2) && __float_as_int(fm) == __float_as_int(L2);
-          // tie-only tap of smallest product f*w
-          const float f = (w >= 0.0f) ? fminf(fp, fm) : fmaxf(fp, fm);
-          fnr = !have_tie ? f : ((w >= 0.0f) ? fminf(fnr, f) : fmaxf(fnr, f));
-          have_tie = true;
-        } else {
-          ok = false;
-        }
-      }
-      if (ok && R <= 2) code = (R + 2) | (have_tie ? kWinHasTieOnly : 0) | ((have_tie && tie_l2) ? kWinTieIsL2 : 0);
-    }
-    tile[(a.Lv + 1) * 33 + lane] = fnr;
-    tile[(a.Lv + 2) * 33 + lane] = __int_as_float(code);
+    classify_taps(a, tile, lane);
   }
+}
+
+// The taps and edge weights of block b copied straight into a tile (4-byte
+// cp.async, one group), without registers held for the 32 steps in between.
+template <typename T>
+__device__ __forceinline__ void stage_taps(const FwdArgs& a, const Chain<T>& c, int b, int lane, int nsteps,
+                                           float* tile) {
+  const int i = 32 * b + lane;
+  if (i < nsteps) {
+    const int64_t HW = static_cast<int64_t>(a.H) * a.W;
+    const int pin = c.pin0 + i * c.dpin;
+    const int ne = (a.eb == 1) ? 0 : c.n, nj = (a.jb == 1) ? 0 : c.n;
+    cp_async4(tile + a.Lv * 33 + lane, a.edge + (static_cast<int64_t>(ne) * 4 + c.dir) * HW + pin);
+    const float* src = static_cast<const float*>(a.jump) + ((static_cast<int64_t>(nj) * 4 + c.dir) * a.Lv) * HW + pin;
+    for (int k = 0; k < a.Lv; ++k) cp_async4(tile + k * 33 + lane, src + static_cast<int64_t>(k) * HW);
+  }
+  cp_async_commit();
+}
+
+// Lean form of a sender (float storage), for the step that runs without a
+// branch per label.  It holds where w > 0 and L2 > 0 are finite, the offset
+// and the own-label tap are 0, and every other tap inside the window is
+// either below L2 with |jd| <= 2 or bitwise L2.  A tap that is bitwise L2
+// gives the candidate's own value at the sender of the minimum and more
+// everywhere else (unless another sender reaches the candidate, which the
+// step tests), so it changes neither value nor argmin and is left out: its
+// entry is +inf, like the entry of an offset outside the window.
+// Record: {w, L2, f(t-1), f(t+1)} and {f(t-2), f(t+2)}, f(s) the tap of
+// sender s; -w in place of w where a tap at distance 2 is below L2 (the wide
+// form), 0 where the form does not hold.
+__device__ __forceinline__ void store_lean(const FwdArgs& a, float* tile, int lane) {
+  const float kInf = __int_as_float(0x7f800000), kMax = __int_as_float(0x7f7fffff);
+  const int c0 = a.Lv / 2;
+  const float w = tile[a.Lv * 33 + lane];
+  const float L2 = tile[(a.Lv - 1) * 33 + lane];
+  bool ok = tile[lane] == 0.0f && a.delta <= kFastDelta && a.delta < a.L && tile[c0 * 33 + lane] == 0.0f && w > 0.0f &&
+            w < kInf && L2 > 0.0f && L2 < kInf;
+  float f[4] = {kInf, kInf, kInf, kInf};  // senders t-2, t-1, t+1, t+2
+#pragma unroll
+  for (int q = 1; q <= kFastDelta; ++q) {
+    if (q > a.delta) break;
+    const float fp = tile[max(1, c0 - q) * 33 + lane];          // sender t+q
+    const float fm = tile[min(a.Lv - 1, c0 + q) * 33 + lane];  // sender t-q
+    const bool bp = fp < L2 && fp >= -kMax, bm = fm < L2 && fm >= -kMax;
+    const bool tp = __float_as_int(fp) == __float_as_int(L2), tm = __float_as_int(fm) == __float_as_int(L2);
+    ok = ok && (bp || tp) && (bm || tm) && (q <= 2 || (tp && tm));
+    if (q == 1) {
+      f[1] = bm ? fm : kInf;
+      f[2] = bp ? fp : kInf;
+    } else if (q == 2) {
+      f[0] = bm ? fm : kInf;
+      f[3] = bp ? fp : kInf;
+    }
+  }
+  float* rec = tile + lean_off(a.Lv);
+  const bool wide = fminf(f[0], f[3]) < kInf;
+  reinterpret_cast<float4*>(rec)[lane] = make_float4(ok ? (wide ? -w : w) : 0.0f, L2, f[1], f[2]);
+  reinterpret_cast<float2*>(rec + 128)[lane] = make_float2(f[0], f[3]);
 }
 
 // Barrier over the NW warps of one chain (named barrier `id`), returning the
@@ -357,9 +442,32 @@ constexpr int kHiOcc = 17;
 template <int OCC>
 constexpr int fwd_block_warps() { return (OCC > 1) ? 1 : 4; }
 
-template <int K, int VARIANT, int NW, typename T, int OCC>
+// min over a lane's label slots
+template <int K>
+__device__ __forceinline__ float slot_min(const float (&v)[K]) {
+  float m[K];
+#pragma unroll
+  for (int k = 0; k < K; ++k) m[k] = v[k];
+#pragma unroll
+  for (int n = K; n > 1; n = (n + 2) / 3) {
+#pragma unroll
+    for (int k = 0; k < (n + 2) / 3; ++k)
+      m[k] = (3 * k + 2 < n) ? fmin3(m[3 * k], m[3 * k + 1], m[(3 * k + 2 < n) ? 3 * k + 2 : 0])
+             : (3 * k + 1 < n) ? fminf(m[3 * k], m[(3 * k + 1 < n) ? 3 * k + 1 : 0]) : m[3 * k];
+  }
+  return m[0];
+}
+
+// The instantiations whose step has the lean form (see store_lean).
+template <int K, int VARIANT, int NW, typename T>
+constexpr bool fwd_lean = VARIANT == BPL_LBP_STEREO && sizeof(T) == 4 && NW == 1 && K <= 8;
+
+// PH: the phase (a.phase) when known at compile time, else -1.
+template <int K, int VARIANT, int NW, typename T, int OCC, int PH = -1>
 __global__ void __launch_bounds__(32 * fwd_block_warps<OCC>(), OCC) lbp_forward_kernel(FwdArgs a) {
   constexpr bool kExact = sizeof(T) == 4;  // float storage: the reference's exact arithmetic
+  constexpr bool kLean = fwd_lean<K, VARIANT, NW, T>;
+  const int phase = (PH < 0) ? a.phase : PH;
   static_assert(K % NW == 0, "labels must split evenly over the chain's warps");
   static_assert(NW == 1 || VARIANT != BPL_LBP_SEM_PIXEL, "pixel variant runs one warp per chain");
   constexpr int KW = K / NW;
@@ -384,7 +492,7 @@ __global__ void __launch_bounds__(32 * fwd_block_warps<OCC>(), OCC) lbp_forward_
   }
   WarpSmem sm;
   {
-    float* p = smem + cpb * chain_smem_floats(K) + wib * warp_smem_floats(a.ns, lroww, a.lmat, a.Lv, sizeof(T));
+    float* p = smem + cpb * chain_smem_floats(K) + wib * warp_smem_floats(a.ns, lroww, a.lmat, a.Lv, sizeof(T), kLean);
     sm.ring = p;
     p += ring_floats(a.ns, lroww, a.lmat, sizeof(T));
     sm.bars = reinterpret_cast<uint64_t*>(p);
@@ -413,7 +521,7 @@ __global__ void __launch_bounds__(32 * fwd_block_warps<OCC>(), OCC) lbp_forward_
   int len;
   {
     const int r = chain_id >> 1;
-    if (a.phase == 0) {
+    if (phase == 0) {
       c.dir = (chain_id & 1) ? LEFT : RIGHT;
       c.n = r / a.H;
       const int y = r % a.H;
@@ -432,8 +540,8 @@ __global__ void __launch_bounds__(32 * fwd_block_warps<OCC>(), OCC) lbp_forward_
   const int nsteps = len - 1;
   if (nsteps <= 0) return;
   const int od = c.dir ^ 1;
-  const int sa = (a.phase == 0) ? UP : RIGHT;
-  const int sb = (a.phase == 0) ? DOWN : LEFT;
+  const int sa = (phase == 0) ? UP : RIGHT;
+  const int sb = (phase == 0) ? DOWN : LEFT;
   c.cost = static_cast<const T*>(a.cost) + static_cast<int64_t>(c.n) * HWL;
   c.slot_a = static_cast<const T*>(a.msgs) + (static_cast<int64_t>(c.n) * 4 + sa) * HWL;
   c.slot_b = static_cast<const T*>(a.msgs) + (static_cast<int64_t>(c.n) * 4 + sb) * HWL;
@@ -485,7 +593,27 @@ __global__ void __launch_bounds__(32 * fwd_block_warps<OCC>(), OCC) lbp_forward_
   constexpr bool kPixGlobal = (VARIANT == BPL_LBP_SEM_PIXEL) && !kRing;
   const int G = kRing ? a.sps : 1;
   T ncst[KW], nva[KW], nvb[KW];  // raw: converted when used, so the loads do not stall here
+  // lean: running pointers (this lane's label 0 of the next step's rows)
+  const T* pc = c.cost + static_cast<int64_t>(c.pin0) * Ls + lane;
+  const T* pa = c.slot_a + static_cast<int64_t>(c.pin0) * Ls + lane;
+  const T* pb = c.slot_b + static_cast<int64_t>(c.pin0) * Ls + lane;
+  const int64_t pstep = static_cast<int64_t>(c.dpin) * Ls;
+  if constexpr (kLean) ncst[KW - 1] = nva[KW - 1] = nvb[KW - 1] = T(0.0f);
   auto prefetch = [&](int i) {
+    if constexpr (kLean) {
+#pragma unroll
+      for (int kk = 0; kk < KW; ++kk) {
+        if (lvalid(kk)) {
+          ncst[kk] = __ldg(pc + 32 * kk);
+          nva[kk] = __ldg(pa + 32 * kk);
+          nvb[kk] = __ldg(pb + 32 * kk);
+        }
+      }
+      pc += pstep;
+      pa += pstep;
+      pb += pstep;
+      return;
+    }
     const int64_t po = static_cast<int64_t>(c.pin0 + i * c.dpin) * Ls;
 #pragma unroll
     for (int kk = 0; kk < KW; ++kk) {
@@ -522,21 +650,237 @@ __global__ void __launch_bounds__(32 * fwd_block_warps<OCC>(), OCC) lbp_forward_
     }
   }
 
+  const int delta = a.delta;
+  const int tile_stride = tap_tile_floats(a.Lv, kLean);
   TapRegs tr;
-  load_taps(a, c, 0, lane, nsteps, tr, stereo);
-  store_taps(a, sm.taps, lane, tr, stereo);
-  if (nsteps > 32) load_taps(a, c, 1, lane, nsteps, tr, stereo);
+  if constexpr (kLean) {
+    stage_taps(a, c, 0, lane, nsteps, sm.taps);
+    cp_async_wait<0>();
+    classify_taps(a, sm.taps, lane);
+    store_lean(a, sm.taps, lane);
+    if (nsteps > 32) stage_taps(a, c, 1, lane, nsteps, sm.taps + tile_stride);
+  } else {
+    load_taps(a, c, 0, lane, nsteps, tr, stereo);
+    store_taps(a, sm.taps, lane, tr, stereo);
+    if (nsteps > 32) load_taps(a, c, 1, lane, nsteps, tr, stereo);
+  }
   __syncwarp();
 
-  const int delta = a.delta;
-  const int tile_stride = tap_tile_rows(a.Lv) * 33;
   const int sf = stage_elems(lroww, a.lmat);
   const float kInf = __int_as_float(0x7f800000);
   bool failed = false;
   int st = 0;
   uint32_t par = 0;
   int pin = c.pin0;
+  // the argmin row at element offset qo of the slot
+  auto store_argmin = [&](const int (&am)[KW], int64_t qo) {
+    const int64_t ao = c.out_off + qo;
+    if (a.argmin_kind == BPL_ARGMIN_U8) {
+      uint8_t* d = static_cast<uint8_t*>(a.argmin) + ao;
+#pragma unroll
+      for (int kk = 0; kk < KW; ++kk)
+        if (lvalid(kk)) d[c.t0 + lane + 32 * kk] = static_cast<uint8_t>(am[kk]);
+    } else if (a.argmin_kind == BPL_ARGMIN_U16) {
+      uint16_t* d = static_cast<uint16_t*>(a.argmin) + ao;
+#pragma unroll
+      for (int kk = 0; kk < KW; ++kk)
+        if (lvalid(kk)) d[c.t0 + lane + 32 * kk] = static_cast<uint16_t>(am[kk]);
+    } else if (a.argmin_kind == BPL_ARGMIN_F32) {
+      float* d = static_cast<float*>(a.argmin) + ao;
+#pragma unroll
+      for (int kk = 0; kk < KW; ++kk)
+        if (lvalid(kk)) d[c.t0 + lane + 32 * kk] = static_cast<float>(am[kk]);
+    }
+  };
+  // next tap block, after the last step of block b
+  auto next_block = [&](int b) {
+    __syncwarp();
+    if (32 * (b + 1) < nsteps) {
+      float* next = sm.taps + ((b + 1) & 1) * tile_stride;
+      if constexpr (kLean) {
+        cp_async_wait<0>();
+        classify_taps(a, next, lane);
+        store_lean(a, next, lane);
+        // (every lane is past its reads of block b's tile: the __syncwarp above)
+        if (32 * (b + 2) < nsteps) stage_taps(a, c, b + 2, lane, nsteps, sm.taps + (b & 1) * tile_stride);
+      } else {
+        store_taps(a, next, lane, tr, stereo);
+        if (32 * (b + 2) < nsteps) load_taps(a, c, b + 2, lane, nsteps, tr, stereo);
+      }
+    }
+    __syncwarp();
+  };
   for (int i = 0; i < nsteps; ++i, pin += c.dpin) {
+    float h[KW], pm;
+    float msg[KW];
+    int am[KW];
+    float e[KW];
+    // kLean, when the hot loop stops: the step can run the dense form below
+    bool lean_dense = false;
+    if constexpr (kLean) {
+      // Hot loop (see store_lean): one straight-line block from h to the
+      // logarithm of the sum, each lane evaluating one exp (its one label
+      // below the candidate, or the candidate's) and one vote at the end
+      // covering everything that would need more, so that nothing on the
+      // dependency chain waits for a branch.  It stops at a step with a
+      // second sender within rounding of the candidate, a window term equal
+      // to the candidate or to 0 (ties and their signs), several labels
+      // below the candidate in a lane or one in every lane, a rounding of
+      // exp or log that is undecided, a NaN or infinity, or a record of
+      // another form; that step runs the code after the loop, which is kept
+      // out of the hot loop's way.  WIDE: taps at distance 2 below L2.
+      // (Moving the stores and the next step's h before the vote, to overlap
+      // it, gained 2 % on the latency-bound launch and lost 3 % on the
+      // others.)
+      auto hot = [&](auto WIDE) {
+        constexpr bool kWide = decltype(WIDE)::value;
+        const float* blk = sm.taps + ((i >> 5) & 1) * tile_stride + lean_off(a.Lv);
+        const float4* rec = reinterpret_cast<const float4*>(blk) + (i & 31);
+        const float2* rec2 = reinterpret_cast<const float2*>(blk + 128) + (i & 31);
+        int left = min(32 - (i & 31), nsteps - i);  // steps to the end of the block or scanline
+        const bool am_wide = a.argmin_kind == BPL_ARGMIN_U8 && a.am_vec == 16;
+        const bool am_other = a.argmin_kind != BPL_ARGMIN_NONE && !am_wide;
+        const bool fills = am_wide && lane < (L >> 4);
+        const int64_t q0 = static_cast<int64_t>(pin + c.dpin) * Ls;
+        T* pd = c.slot_out + q0 + lane;
+        uint8_t* arow = static_cast<uint8_t*>(a.argmin) + (c.out_off + q0);
+        float* psc = scale_out + pin + c.dpin;
+        // The rows of the step kL2Ahead further on, brought into L2 by one
+        // instruction (lane: one 128-byte line of a row): the register
+        // prefetch one step ahead then meets L2 latency instead of DRAM's.
+        // With few warps per SM (horizontal launch at 188x620x96 0.41 ->
+        // 0.37 ms), and down the columns where the resident warps' rows are
+        // too few bytes in flight for DRAM (17 warps x 3 rows x 384 bytes;
+        // vertical launch at 4x256x512x96 0.43 -> 0.35 ms).  At 192 labels
+        // the vertical launch already streams at 80 % of the copy rate and
+        // it costs 5 %; along rows with 13 warps per SM it costs 4 %.
+        constexpr bool kAhead = OCC == 1 || (PH == 1 && K <= 4);
+        const int prow = lane / (K + 1), pline = lane % (K + 1);
+        const bool pf_lane = prow < 3 && 32 * pline < L;
+        const char* ppf = reinterpret_cast<const char*>((prow == 1 ? c.slot_a : prow == 2 ? c.slot_b : c.cost) +
+                                                        (static_cast<int64_t>(pin) + min(kL2Ahead, nsteps - 1 - i) * c.dpin) * Ls) +
+                          (pf_lane ? 128 * pline : 0);
+        for (;;) {
+          const float4 lt = *rec;
+          const float w = kWide ? -lt.x : lt.x;
+#pragma unroll
+          for (int kk = 0; kk < KW; ++kk) {
+            const float hv = (phase == 0) ? __fadd_rn(__fadd_rn(__fadd_rn(ncst[kk], chain[kk]), nva[kk]), nvb[kk])
+                                          : __fadd_rn(__fadd_rn(__fadd_rn(ncst[kk], nva[kk]), nvb[kk]), chain[kk]);
+            h[kk] = lvalid(kk) ? hv : kInf;
+            cs.hs[lane + 32 * kk] = h[kk];
+          }
+          pm = warp_min_f32(slot_min<KW>(h));
+          __syncwarp();
+          // (a branch of its own: loads in the block itself are moved down
+          // towards their use, and their latency with them; horizontal
+          // launch at 376x1240x192 0.99 ms without it)
+          if (i + 1 < nsteps) prefetch(i + 1);
+          if (kAhead) {
+            prefetch_l2(ppf);
+            ppf += (i + kL2Ahead + 1 < nsteps) ? pstep * static_cast<int64_t>(sizeof(T)) : 0;
+          }
+          float mw[KW];
+#pragma unroll
+          for (int kk = 0; kk < KW; ++kk) {
+            const float* hk = cs.hs + lane + 32 * kk;
+            mw[kk] = fmin3(__fmaf_rn(lt.z, w, hk[-1]), h[kk], __fmaf_rn(lt.w, w, hk[1]));
+          }
+          float2 l2;
+          if constexpr (kWide) {
+            l2 = *rec2;
+#pragma unroll
+            for (int kk = 0; kk < KW; ++kk) {
+              const float* hk = cs.hs + lane + 32 * kk;
+              mw[kk] = fmin3(__fmaf_rn(l2.x, w, hk[-2]), mw[kk], __fmaf_rn(l2.y, w, hk[2]));
+            }
+          }
+          // Counts (in units of 2^16) and slots of the senders within
+          // rounding of the candidate's (at most 2^-21 (|pm| + L2 w) above the
+          // minimum, four times the spacing of the candidates' floats; the
+          // minimum itself is one) and of the labels below the candidate.
+          const float msg_g = __fmaf_rn(lt.y, w, pm);
+          const float thr = __fmaf_rn(__fmaf_rn(lt.y, w, fabsf(pm)), 4.76837158203125e-07f, pm);
+          int near = 0, own = 0;
+          float m[KW];
+#pragma unroll
+          for (int kk = 0; kk < KW; ++kk) {
+            if (h[kk] <= thr) near += 0x10000 + 32 * kk;
+            if (lvalid(kk) && mw[kk] <= msg_g) own += 0x10000 + 32 * kk;
+            m[kk] = fminf(mw[kk], msg_g);
+            if (!lvalid(kk)) m[kk] = msg_g;
+          }
+          const unsigned nearl = __ballot_sync(FULL, near != 0);
+          const unsigned ownl = __ballot_sync(FULL, own != 0);
+          const float xs = slot_min<KW>(m);
+          float y;
+          const bool okx = crm::exp_fast(xs, y, s_exp);
+          const float e_g = __shfl_sync(FULL, y, __ffs(~ownl) - 1);
+          float ev[K];
+#pragma unroll
+          for (int kk = 0; kk < KW; ++kk) {
+            ev[kk] = (m[kk] == msg_g) ? e_g : y;
+            if (!lvalid(kk)) ev[kk] = 0.0f;
+          }
+          // argmin of h, and of this lane's label (the last minimiser in
+          // sender order)
+          const int argmin_h = __reduce_max_sync(FULL, near != 0 ? (near & 0xffff) + lane : -1);
+          const bool owns = (own >> 16) == 1;  // (several labels: the vote fails)
+          const int t = lane + (own & 0xe0);
+          int arg = (cs.hs[t] == xs) ? t : t - 1;
+          if constexpr (kWide) arg = (arg == t || __fmaf_rn(lt.z, w, cs.hs[t - 1]) == xs) ? arg : t - 2;
+          arg = (__fmaf_rn(lt.w, w, cs.hs[t + 1]) == xs) ? t + 1 : arg;
+          if constexpr (kWide) arg = (__fmaf_rn(l2.y, w, cs.hs[t + 2]) == xs) ? t + 2 : arg;
+          const bool form = w > 0.0f;
+          const bool near1 = near < 0x20000 && (nearl & (nearl - 1u)) == 0u && nearl != 0u;
+          const float sum = tree_sum<K>(ev);
+          float lse;
+          const bool okl = crm::log_fast(sum, lse, s_log);
+          const bool good = form && near1 && own < 0x20000 && ownl != FULL && okx && okl &&
+                            (own == 0 || (xs != msg_g && xs != 0.0f));
+          if (!__all_sync(FULL, good)) {
+            lean_dense = __all_sync(FULL, form && near1);
+            return;
+          }
+#pragma unroll
+          for (int kk = 0; kk < KW; ++kk) {
+            chain[kk] = __fsub_rn(m[kk], lse);
+            if (lvalid(kk)) pd[32 * kk] = chain[kk];
+          }
+          if (lane == 0) *psc = sum;
+          // uint8 argmin rows of whole 16-byte chunks: filled with the
+          // minimum's label, then the few other labels' bytes
+          const unsigned f4 = static_cast<unsigned>(argmin_h) * 0x01010101u;
+          if (fills) reinterpret_cast<uint4*>(arow)[lane] = make_uint4(f4, f4, f4, f4);
+          __syncwarp();  // (also: hs is rewritten by the next step)
+          if (am_wide && owns) arow[t] = static_cast<uint8_t>(arg);
+          if (am_other) {
+            int am[KW];
+#pragma unroll
+            for (int kk = 0; kk < KW; ++kk) am[kk] = (owns && t == lane + 32 * kk) ? arg : argmin_h;
+            store_argmin(am, static_cast<int64_t>(pin + c.dpin) * Ls);
+          }
+          ++i;
+          pin += c.dpin;
+          pd += pstep;
+          arow += pstep;
+          psc += c.dpin;
+          ++rec;
+          if constexpr (kWide) ++rec2;
+          if (--left == 0) {
+            if (i == nsteps) return;
+            next_block((i >> 5) - 1);
+            blk = sm.taps + ((i >> 5) & 1) * tile_stride + lean_off(a.Lv);
+            rec = reinterpret_cast<const float4*>(blk);
+            rec2 = reinterpret_cast<const float2*>(blk + 128);
+            left = min(32, nsteps - i);
+          }
+        }
+      };
+      if (sm.taps[((i >> 5) & 1) * tile_stride + lean_off(a.Lv) + 4 * (i & 31)] < 0.0f) hot(std::true_type{});
+      else hot(std::false_type{});
+      if (i == nsteps) break;
+    }
     const int j = i & 31;
     const int b = i >> 5;
     const float* tile = sm.taps + (b & 1) * tile_stride;
@@ -574,59 +918,97 @@ __global__ void __launch_bounds__(32 * fwd_block_warps<OCC>(), OCC) lbp_forward_
       __syncwarp();
     }
 
-    // h = cost + incoming messages except the chain direction's own slot,
-    // added in the reference order RIGHT, LEFT, UP, DOWN.
-    float h[KW];
+    if constexpr (!kLean) {
+      // h = cost + incoming messages except the chain direction's own slot,
+      // added in the reference order RIGHT, LEFT, UP, DOWN.
 #pragma unroll
-    for (int kk = 0; kk < KW; ++kk) {
-      // branch-free: the ring rows are lroww long; labels >= L read padding
-      // and get +inf (never a minimum)
-      const int tl = lane + 32 * kk;  // label within the warp's range
-      const float cst = ldf<T>(kRing ? stg[tl] : ncst[kk]);
-      const float va = ldf<T>(kRing ? stg[lroww + tl] : nva[kk]);
-      const float vb = ldf<T>(kRing ? stg[2 * lroww + tl] : nvb[kk]);
-      const float hv = (a.phase == 0) ? __fadd_rn(__fadd_rn(__fadd_rn(cst, chain[kk]), va), vb)
-                                      : __fadd_rn(__fadd_rn(__fadd_rn(cst, va), vb), chain[kk]);
-      h[kk] = lvalid(kk) ? hv : kInf;
-      cs.hs[c.t0 + tl] = h[kk];
-    }
-    // partial minimum over the warp's labels (one redux), with its tie count
-    // and, when the minimum is unique, its label
-    float pm = h[0];
+      for (int kk = 0; kk < KW; ++kk) {
+        // branch-free: the ring rows are lroww long; labels >= L read padding
+        // and get +inf (never a minimum)
+        const int tl = lane + 32 * kk;  // label within the warp's range
+        const float cst = ldf<T>(kRing ? stg[tl] : ncst[kk]);
+        const float va = ldf<T>(kRing ? stg[lroww + tl] : nva[kk]);
+        const float vb = ldf<T>(kRing ? stg[2 * lroww + tl] : nvb[kk]);
+        const float hv = (phase == 0) ? __fadd_rn(__fadd_rn(__fadd_rn(cst, chain[kk]), va), vb)
+                                        : __fadd_rn(__fadd_rn(__fadd_rn(cst, va), vb), chain[kk]);
+        h[kk] = lvalid(kk) ? hv : kInf;
+        cs.hs[c.t0 + tl] = h[kk];
+      }
+      // partial minimum over the warp's labels (one redux), with its tie count
+      // and, when the minimum is unique, its label
+      pm = h[0];
 #pragma unroll
-    for (int kk = 1; kk < KW; ++kk) pm = fminf(pm, h[kk]);
-    pm = warp_min_redux(pm);
-    int lcnt = 0, llab = 0;
+      for (int kk = 1; kk < KW; ++kk) pm = fminf(pm, h[kk]);
+      pm = warp_min_redux(pm);
+    }
+    int pcnt = 0, plab = 0;
+    auto count_min = [&]() {
+      int lcnt = 0, llab = 0;
 #pragma unroll
-    for (int kk = 0; kk < KW; ++kk) {
-      const bool eq = h[kk] == pm;
-      lcnt += eq ? 1 : 0;
-      llab = eq ? c.t0 + lane + 32 * kk : llab;
-    }
-    const int pcnt = __reduce_add_sync(FULL, lcnt);
-    const int plab = __reduce_max_sync(FULL, llab);
-    if (NW > 1 && lane == 0) {
-      cs.red[wic] = pm;
-      reinterpret_cast<int*>(cs.red)[4 + wic] = pcnt;
-      reinterpret_cast<int*>(cs.red)[8 + wic] = plab;
-    }
-    __syncwarp();
-    if (!kRing && i + 1 < nsteps) prefetch(i + 1);
-    // h of the whole pixel and the partial minima are visible to the chain
-    if (NW == 1) {
-      if (!__all_sync(FULL, ok)) {
+      for (int kk = 0; kk < KW; ++kk) {
+        const bool eq = h[kk] == pm;
+        lcnt += eq ? 1 : 0;
+        llab = eq ? c.t0 + lane + 32 * kk : llab;
+      }
+      pcnt = __reduce_add_sync(FULL, lcnt);
+      plab = __reduce_max_sync(FULL, llab);
+    };
+    // kLean: several labels below the candidate in a lane: one exp per label
+    // slot, evaluated side by side
+    bool dense = false;
+    if constexpr (kLean) {
+      if (lean_dense) {
+        const float* rec = tile + lean_off(a.Lv);
+        const float4 lt = reinterpret_cast<const float4*>(rec)[j];
+        const float2 l2 = reinterpret_cast<const float2*>(rec + 128)[j];
+        const float wt = fabsf(lt.x);
+        const float msg_g = __fmaf_rn(lt.y, wt, pm);
+        int near = -1;
+#pragma unroll
+        for (int kk = 0; kk < KW; ++kk) near = (h[kk] == pm) ? lane + 32 * kk : near;
+        const int argmin_h = __reduce_max_sync(FULL, near);
+        bool bad = false;
+#pragma unroll
+        for (int kk = 0; kk < KW; ++kk) {
+          const float* hk = cs.hs + lane + 32 * kk;
+          // senders t-2 .. t+2; the last minimiser wins
+          const float n[5] = {__fmaf_rn(l2.x, wt, hk[-2]), __fmaf_rn(lt.z, wt, hk[-1]), h[kk],
+                              __fmaf_rn(lt.w, wt, hk[1]), __fmaf_rn(l2.y, wt, hk[2])};
+          const float m = fmin3(fmin3(n[0], n[1], n[2]), n[3], n[4]);
+          int arg = lane + 32 * kk - 2;
+#pragma unroll
+          for (int q = 1; q < 5; ++q) arg = (n[q] == m) ? lane + 32 * kk + q - 2 : arg;
+          msg[kk] = fminf(m, msg_g);
+          am[kk] = (m <= msg_g) ? arg : argmin_h;
+          const bool ok_k = crm::exp_fast(msg[kk], e[kk], s_exp);
+          bad = bad || (lvalid(kk) && (!ok_k || m == msg_g || (m < msg_g && m == 0.0f)));
+          if (!lvalid(kk)) e[kk] = 0.0f;
+        }
+        dense = !__any_sync(FULL, bad);
+      }
+      if (!dense) count_min();
+    } else {
+      count_min();
+      if (NW > 1 && lane == 0) {
+        cs.red[wic] = pm;
+        reinterpret_cast<int*>(cs.red)[4 + wic] = pcnt;
+        reinterpret_cast<int*>(cs.red)[8 + wic] = plab;
+      }
+      __syncwarp();
+      if (!kRing && i + 1 < nsteps) prefetch(i + 1);
+      // h of the whole pixel and the partial minima are visible to the chain
+      if (NW == 1) {
+        if (!__all_sync(FULL, ok)) {
+          failed = true;
+          break;
+        }
+      } else if (!chain_sync_and<NW>(bar_id, ok)) {
         failed = true;
         break;
       }
-    } else if (!chain_sync_and<NW>(bar_id, ok)) {
-      failed = true;
-      break;
     }
 
     const float w = tile[a.Lv * 33 + j];
-    float msg[KW];
-    int am[KW];
-    float e[KW];
     // Half storage keeps every message relative to the minimum of h (the
     // labels near the row's minimum, the ones the beliefs depend on, get
     // half's finest steps; a log-normalised row sits near -log L, where a
@@ -643,7 +1025,9 @@ __global__ void __launch_bounds__(32 * fwd_block_warps<OCC>(), OCC) lbp_forward_
     }
     auto earg = [ref](float x) { return kExact ? x : __fsub_rn(x, ref); };
 
-    if (kPcolRegs && delta >= L) {
+    if (kLean && dense) {
+      // (msg, am and e are set)
+    } else if (kPcolRegs && delta >= L) {
       // full minimisation with the register column (see kPcolRegs); same
       // order and tie rule as below.  The 32 senders run as four
       // independent chains over the contiguous ranges [8c, 8c+8), combined
@@ -1090,37 +1474,11 @@ __global__ void __launch_bounds__(32 * fwd_block_warps<OCC>(), OCC) lbp_forward_
       chain[kk] = ldf<T>(o);  // the stored value, so the chain matches memory
       if (lvalid(kk)) dstm[t] = o;
     }
-    {
-      const int64_t ao = c.out_off + qo;
-      if (a.argmin_kind == BPL_ARGMIN_U8) {
-        uint8_t* d = static_cast<uint8_t*>(a.argmin) + ao;
-#pragma unroll
-        for (int kk = 0; kk < KW; ++kk)
-          if (lvalid(kk)) d[c.t0 + lane + 32 * kk] = static_cast<uint8_t>(am[kk]);
-      } else if (a.argmin_kind == BPL_ARGMIN_U16) {
-        uint16_t* d = static_cast<uint16_t*>(a.argmin) + ao;
-#pragma unroll
-        for (int kk = 0; kk < KW; ++kk)
-          if (lvalid(kk)) d[c.t0 + lane + 32 * kk] = static_cast<uint16_t>(am[kk]);
-      } else if (a.argmin_kind == BPL_ARGMIN_F32) {
-        float* d = static_cast<float*>(a.argmin) + ao;
-#pragma unroll
-        for (int kk = 0; kk < KW; ++kk)
-          if (lvalid(kk)) d[c.t0 + lane + 32 * kk] = static_cast<float>(am[kk]);
-      }
-    }
+    store_argmin(am, qo);
     // (float)max((double)sum, 1e-45): the smallest positive float when sum is 0
     if (wic == 0 && lane == 0 && scale_out) scale_out[pq] = (sum > 0.0f) ? sum : __int_as_float(1);
 
-    // next tap block
-    if (j == 31 || i == nsteps - 1) {
-      __syncwarp();
-      if (32 * (b + 1) < nsteps) {
-        store_taps(a, sm.taps + ((b + 1) & 1) * tile_stride, lane, tr, stereo);
-        if (32 * (b + 2) < nsteps) load_taps(a, c, b + 2, lane, nsteps, tr, stereo);
-      }
-      __syncwarp();
-    }
+    if (j == 31 || i == nsteps - 1) next_block(b);
     if (kRing && ++st == a.ns) st = 0;
   }
 
@@ -1139,6 +1497,7 @@ __global__ void __launch_bounds__(32 * fwd_block_warps<OCC>(), OCC) lbp_forward_
 template <int K, int V, int NW, typename T>
 int launch_phase(const FwdArgs& a0, cudaStream_t stream) {
   FwdArgs a = a0;
+  constexpr bool kLean = fwd_lean<K, V, NW, T>;
   const int lroww = 32 * (K / NW);
   if (V == BPL_LBP_SEM_PIXEL && NW == 1 && a.ns > 0 && a.nchains > kHiOccChainsPerSm * sm_count()) {
     // one-warp blocks: the deepest ring (4..2 steps) whose shared memory lets
@@ -1146,7 +1505,7 @@ int launch_phase(const FwdArgs& a0, cudaStream_t stream) {
     // wave of full-length scanlines costs more than a shallower prefetch
     for (int ns = a.ns; ns >= 2; --ns) {
       const size_t pc = 4 * (static_cast<size_t>(chain_smem_floats(K)) +
-                             static_cast<size_t>(warp_smem_floats(ns, lroww, a.lmat, a.Lv, sizeof(T))));
+                             static_cast<size_t>(warp_smem_floats(ns, lroww, a.lmat, a.Lv, sizeof(T), false)));
       const size_t tabs = (sizeof(T) == 4) ? sizeof(crm::Tables) : 0;
       const int per_sm = std::min(32, static_cast<int>(smem_per_sm() / (pc + tabs + smem_reserved_per_block())));
       a.ns = ns;
@@ -1154,16 +1513,19 @@ int launch_phase(const FwdArgs& a0, cudaStream_t stream) {
     }
   }
   const size_t per_chain = 4 * (static_cast<size_t>(chain_smem_floats(K)) +
-                                static_cast<size_t>(NW) * warp_smem_floats(a.ns, lroww, a.lmat, a.Lv, sizeof(T)));
+                                static_cast<size_t>(NW) * warp_smem_floats(a.ns, lroww, a.lmat, a.Lv, sizeof(T), kLean));
   // a phase with more scanlines than about 8 warps per SM runs 1-warp
   // blocks, kHiOcc resident per SM (registers capped near 120); fewer
   // scanlines run latency-bound in 4-warp blocks and keep every register
   // they use
-  auto kern = lbp_forward_kernel<K, V, NW, T, 1>;
+  // (the lean step is compiled per phase: h is summed in another order)
+  constexpr int P0 = kLean ? 0 : -1, P1 = kLean ? 1 : -1;
+  auto kern = (a.phase == 0) ? lbp_forward_kernel<K, V, NW, T, 1, P0> : lbp_forward_kernel<K, V, NW, T, 1, P1>;
   int wmax = 4;
   if constexpr (K <= 8) {
     if (NW == 1 && a.nchains > kHiOccChainsPerSm * sm_count()) {
-      kern = lbp_forward_kernel<K, V, NW, T, kHiOcc>;
+      kern = (a.phase == 0) ? lbp_forward_kernel<K, V, NW, T, kHiOcc, P0>
+                            : lbp_forward_kernel<K, V, NW, T, kHiOcc, P1>;
       wmax = fwd_block_warps<kHiOcc>();
     }
   }
@@ -1206,50 +1568,45 @@ int launch_k(const FwdArgs& a0, cudaStream_t stream) {
 
 template <int V, typename T = float>
 int dispatch_k(const FwdArgs& a, cudaStream_t s) {
+  static_assert(V != BPL_LBP_STEREO, "dispatch_stereo");
   const int k = (a.L + 31) / 32;
-  if constexpr (V != BPL_LBP_STEREO) {
-    // semantic variants: one warp per scanline
-    if constexpr (V == BPL_LBP_SEM_PIXEL) {
-      // per-pixel L x L matrices: staged through the ring up to L = 96,
-      // read from global memory above
-      if (k == 1) return launch_k<1, V, 1, 1, T>(a, s);
-      if (k == 2) return launch_k<2, V, 2, 1, T>(a, s);
-      if (k == 3) return launch_k<3, V, 3, 1, T>(a, s);
+  if constexpr (V == BPL_LBP_SEM_PIXEL) {
+    // per-pixel L x L matrices: staged through the ring up to L = 96,
+    // read from global memory above
+    if (k == 1) return launch_k<1, V, 1, 1, T>(a, s);
+    if (k == 2) return launch_k<2, V, 2, 1, T>(a, s);
+    if (k == 3) return launch_k<3, V, 3, 1, T>(a, s);
+    if (k <= 8) return launch_k<8, V, 8, 1, T>(a, s);
+    return launch_k<32, V, 32, 1, T>(a, s);
+  }
+  switch (k) {
+    case 1: return launch_k<1, V, 1, 1, T>(a, s);
+    case 2: return launch_k<2, V, 2, 1, T>(a, s);
+    case 3: return launch_k<3, V, 3, 1, T>(a, s);
+    case 4: return launch_k<4, V, 4, 1, T>(a, s);
+    default:
       if (k <= 8) return launch_k<8, V, 8, 1, T>(a, s);
+      if (k <= 16) return launch_k<16, V, 16, 1, T>(a, s);
       return launch_k<32, V, 32, 1, T>(a, s);
-    }
-    switch (k) {
-      case 1: return launch_k<1, V, 1, 1, T>(a, s);
-      case 2: return launch_k<2, V, 2, 1, T>(a, s);
-      case 3: return launch_k<3, V, 3, 1, T>(a, s);
-      case 4: return launch_k<4, V, 4, 1, T>(a, s);
-      default:
-        if (k <= 8) return launch_k<8, V, 8, 1, T>(a, s);
-        if (k <= 16) return launch_k<16, V, 16, 1, T>(a, s);
-        return launch_k<32, V, 32, 1, T>(a, s);
-    }
-  } else {
-    // (the split-scanline instantiations KS/NS are enabled together with
-    // kSplitChainsPerSm; with it at 0 every phase runs one warp per scanline)
-    switch (k) {
-      case 1: return launch_k<1, V, 1, 1, T>(a, s);
-      case 2: return launch_k<2, V, 2, 1, T>(a, s);
-      case 3: return launch_k<3, V, 3, 1, T>(a, s);
-      case 4: return launch_k<4, V, 4, 1, T>(a, s);
-      case 5: return launch_k<5, V, 5, 1, T>(a, s);
-      case 6: return launch_k<6, V, 6, 1, T>(a, s);
-      case 7: return launch_k<7, V, 7, 1, T>(a, s);
-      case 8: return launch_k<8, V, 8, 1, T>(a, s);
-      default:
-        if (k <= 12) return launch_k<12, V, 12, 1, T>(a, s);
-        if (k <= 16) return launch_k<16, V, 16, 1, T>(a, s);
-        if (k <= 24) return launch_k<24, V, 24, 1, T>(a, s);
-        return launch_k<32, V, 32, 1, T>(a, s);
-    }
   }
 }
 
+// Stereo: the instantiations K = LO .. HI (1 to 8 for every 32 labels, then
+// 12, 16, 24, 32), compiled in several units.
+constexpr int next_k(int k) { return k < 8 ? k + 1 : k == 8 ? 12 : k == 12 ? 16 : k + 8; }
+
+template <typename T, int LO, int HI>
+int dispatch_stereo(const FwdArgs& a, cudaStream_t s) {
+  if constexpr (LO < HI) {
+    if (a.L > 32 * LO) return dispatch_stereo<T, next_k(LO), HI>(a, s);
+  }
+  return launch_k<LO, BPL_LBP_STEREO, LO, 1, T>(a, s);
+}
+
 int lbp_forward_stereo(const FwdArgs& a, cudaStream_t s);
+int lbp_forward_stereo_k5(const FwdArgs& a, cudaStream_t s);
+int lbp_forward_stereo_k7(const FwdArgs& a, cudaStream_t s);
+int lbp_forward_stereo_k12(const FwdArgs& a, cudaStream_t s);
 int lbp_forward_sem_global(const FwdArgs& a, cudaStream_t s);
 int lbp_forward_sem_pixel(const FwdArgs& a, cudaStream_t s);
 int lbp_forward_stereo_f16(const FwdArgs& a, cudaStream_t s);

@@ -6,6 +6,6 @@
 namespace bpl {
 int lbp_forward_stereo_f16(const FwdArgs& a, cudaStream_t s) {
   if (a.L <= 256) return dispatch_f16(a, s);
-  return dispatch_k<BPL_LBP_STEREO, __half>(a, s);
+  return dispatch_stereo<__half, 12, 32>(a, s);
 }
 }  // namespace bpl
