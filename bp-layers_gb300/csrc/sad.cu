@@ -18,14 +18,10 @@
 // summed), and blocks of up to 384 threads run with registers capped so that
 // 2-3 are resident per SM: one block's chunk barrier then leaves the others
 // issuing (a 512-thread block, D > 192, stays alone on its SM).
-// Backward: lanes are channels and each thread owns 4 pixels; both sums walk
-// the disparities in the reference order (additions of +-g in the same
-// sequence: bit-identical).  Per chunk of 32 disparities the block stages
-// (cp.async, double-buffered) its channels' f1 segment x - d, f0 segment
-// x + d and the two gradient tables g[x, d] and g[x + d, d], which the warp
-// reads as broadcasts; the thread slides a register window over its feature
-// rows, so a term is a subtraction, a sign-bit operation, the |diff| test
-// and a predicated add (ALU-pipe bound).
+// Backward: lanes are channels; both sums add +-g in the reference's order
+// (bit-identical) in one pass over the (pixel, disparity) pairs
+// (sad_backward_kernel), or, for few rows, each gathered by its pixel's
+// thread (sad_backward_gather_kernel).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -205,15 +201,288 @@ struct SadBwdArgs {
   const float* g;
   float* df0;
   float* df1;
-  int B, C, H, W, D, min_disp, max_disp;
+  int B, C, H, W, D, min_disp;
+  int Dg, g0;  // disparities of the gradient volume; the first of this launch's D within it
+  int nb;      // f1 blocks a strip meets
+  int accum;   // add to df0 / df1 (a later range of disparities)
   int channel_limit;
 };
 
-constexpr int kBX = 32;            // pixels per block (backward)
-constexpr int kBPX = 4;            // pixels per thread
-constexpr int kBCH = 32;           // channels per block: lane = channel
-constexpr int kBDC = 32;           // disparities per staged chunk
-constexpr int kBFS = kBX + kBDC - 1;  // staged feature row (odd: lanes' rows fall in distinct banks)
+constexpr int kBT = 8;       // pixels per strip and per f1 block
+constexpr int kBWarps = 16;  // strips per block at most
+constexpr int kBGS = 4;      // stages of a strip's gradient tiles
+constexpr int kBMaxD = 256;  // disparities per launch
+constexpr int kBPitch = kBT * kBWarps + 4;  // floats of a staged feature row (lanes' 16-byte reads in distinct banks)
+
+// blocks a strip meets: e = x - u in [8 tau - 7, 8 tau + 7] must reach D - 1
+inline int sad_bwd_blocks(int D) { return (D + 6) / kBT + 1; }
+
+inline size_t sad_bwd_smem_bytes(int strips, int nb) {
+  // hand-over of (f1, df1) blocks between strips (two per strip) and between
+  // segments (nb + 1 slots), 2 KB each, the gradient tiles, and two buffers
+  // of a segment's f0 and f1 rows
+  return (2u * strips + nb + 1u) * 2048u + static_cast<size_t>(strips) * kBGS * kBT * kBT * 4u + 4u * 32u * kBPitch * 4u;
+}
+
+// cp.async of N bytes (4 or 16), zeros when !ok
+template <int N>
+__device__ __forceinline__ void cp_async_or_zero(void* dst, const void* src, bool ok) {
+  const int n = ok ? N : 0;
+  if constexpr (N == 16)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(n) : "memory");
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(n) : "memory");
+}
+
+// One (pixel, matched pixel) pair of both sums: df0 += (diff/|diff|) g and
+// df1 -= (diff/|diff|) g when |diff| > 1e-15.  diff/|diff| is exactly +-1 and
+// its product with g exact, so each update rounds once, like the
+// reference's; a NaN diff never passes the test.
+// (Written in PTX so that both updates are predicated: the compiler's form of
+// the same statements had seven instructions.)
+__device__ __forceinline__ void sad_pair(float v0, float v1, float g, float& a0, float& a1) {
+  asm("{\n"
+      " .reg .f32 d, e, s, t;\n .reg .b32 u;\n .reg .pred p;\n"
+      " sub.rn.f32 d, %2, %3;\n"
+      " abs.f32 e, d;\n"
+      " setp.gt.f32 p, e, 0f26901D7D;\n"  // 1e-15f
+      " mov.b32 u, d;\n"
+      " lop3.b32 u, u, 0x80000000, 0x3f800000, 0xEA;\n"  // (u & sign) | 1.0f
+      " mov.b32 s, u;\n"
+      " neg.f32 t, s;\n"
+      " @p fma.rn.f32 %0, s, %4, %0;\n"
+      " @p fma.rn.f32 %1, t, %4, %1;\n"
+      "}"
+      : "+f"(a0), "+f"(a1)
+      : "f"(v0), "f"(v1), "f"(g));
+}
+
+// Both gradients in one pass over the (pixel, disparity) pairs, each pair's
+// difference, sign and test shared by the two sums it enters.  With
+// u = x' + min_disp (x' the f1 column) a pair has e = d - min_disp = x - u.
+// df0[x] sums over e ascending (u descending), df1[u] over e ascending (x
+// ascending): blocks of 8 x 8 pairs run in exactly that order when strip s
+// (8 pixels, one warp, lane = channel, f0 and df0 in registers) meets the f1
+// blocks s, s-1, s-2, ... and every f1 block, with its running df1, moves
+// from strip to strip to the right.  A block of threads owns one image row
+// and 32 channels; its warps are neighbouring strips in step (one barrier
+// per 64 pairs), blocks pass between them through shared memory, and a row
+// longer than its strips runs in segments from left to right, the blocks
+// that leave a segment kept for the next (slot (tau - 2k) mod (nb + 1) for
+// the one leaving segment k after step tau: the slot read one step before).
+//
+// A pair costs a subtraction, two fused multiply-adds (FMA pipe), a sign
+// merge and a test (ALU pipe, half rate): five issue slots and four ALU
+// cycles, where one pass per sum took eight and eight, and the gradient is
+// read once per 32 channels instead of twice.  376x1240, C = 64, D = 192:
+// 3.48 -> 1.57 ms (70 % of issue slots, ALU pipe 54 %).  grid (H * ceil(C/32), B); block 32 x strips.
+// VEC: gradient rows start on 16-byte boundaries (D and the pointer), copied
+// 16 bytes at a time.
+template <bool VEC>
+__global__ void __launch_bounds__(32 * kBWarps, 1) sad_backward_kernel(SadBwdArgs a) {
+  extern __shared__ __align__(16) float sm[];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, S = blockDim.x >> 5;
+  float4* xfer = reinterpret_cast<float4*>(sm);          // [2][S][4][32]
+  float4* ring = xfer + 2 * S * 128;                     // [nb + 1][4][32]
+  float* gts = reinterpret_cast<float*>(ring + (a.nb + 1) * 128);
+  float* gt = gts + w * kBGS * kBT * kBT;                // [kBGS][8][8] of this strip
+  float* rows = gts + S * kBGS * kBT * kBT;              // [2][f0, f1][32][kBPitch]
+  const int ncb = (a.C + 31) / 32;  // (neighbouring blocks read the same gradient row)
+  const int n = blockIdx.y, y = blockIdx.x / ncb;
+  const int c0 = (blockIdx.x % ncb) * 32;
+  const int c = c0 + lane;
+  const bool cok = c < a.C;
+  const int64_t HW = static_cast<int64_t>(a.H) * a.W;
+  const int64_t plane = static_cast<int64_t>(n) * a.C * HW + static_cast<int64_t>(y) * a.W;
+  const int64_t row = plane + (cok ? c : 0) * HW;
+  const float* f1r = a.f1 + row;
+  float* df0r = a.df0 + row;
+  float* df1r = a.df1 + row;
+  const bool store = cok && c < a.channel_limit;
+  const float* grow = a.g + (static_cast<int64_t>(n) * a.H + y) * a.W * a.Dg + a.g0;
+  const float qnan = __int_as_float(0x7fffffff);
+  const int nb = a.nb, R = nb + 1;
+  const int nstrips = (a.W + kBT - 1) / kBT;
+  const int nseg = (nstrips + S - 1) / S;
+
+  float v1[kBT], acc1[kBT];  // the current f1 block (NaN outside the image) and its df1
+  auto fresh_block = [&](int j) {
+#pragma unroll
+    for (int i = 0; i < kBT; ++i) {
+      const int x = kBT * j + i - a.min_disp;
+      const bool ok = cok && x >= 0 && x < a.W;
+      v1[i] = ok ? __ldg(f1r + x) : qnan;
+      acc1[i] = (ok && a.accum) ? df1r[x] : 0.0f;
+    }
+  };
+  auto store_block = [&](int j) {
+#pragma unroll
+    for (int i = 0; i < kBT; ++i) {
+      const int x = kBT * j + i - a.min_disp;
+      if (store && x >= 0 && x < a.W) df1r[x] = acc1[i];
+    }
+  };
+  // Feature rows and results pass through shared memory, [channel][column]:
+  // global accesses along the row, the lanes' own channels beside them
+  // (lanes on their channels' rows directly cost 32 lines per access: half
+  // of the kernel's time).  Columns x1 .. x1 + 8 S - 1 of the row.
+  auto load_rows = [&](float* dst, const float* src, int x1) {
+    for (int cc = w; cc < 32 && c0 + cc < a.C; cc += S) {
+      const float* sr = src + plane + (c0 + cc) * HW + x1;
+      for (int q = lane; q < kBT * S; q += 32)
+        if (x1 + q >= 0 && x1 + q < a.W) cp_async4(dst + cc * kBPitch + q, sr + q);
+    }
+  };
+  auto store_rows = [&](const float* src, float* dst, int x1, int cols) {
+    for (int cc = w; cc < 32 && c0 + cc < a.channel_limit; cc += S) {
+      float* dr = dst + plane + (c0 + cc) * HW + x1;
+      for (int q = lane; q < cols; q += 32)
+        if (x1 + q >= 0 && x1 + q < a.W) dr[q] = src[cc * kBPitch + q];
+    }
+  };
+  auto put = [&](float4* slot) {
+    slot[lane] = make_float4(v1[0], v1[1], v1[2], v1[3]);
+    slot[32 + lane] = make_float4(v1[4], v1[5], v1[6], v1[7]);
+    slot[64 + lane] = make_float4(acc1[0], acc1[1], acc1[2], acc1[3]);
+    slot[96 + lane] = make_float4(acc1[4], acc1[5], acc1[6], acc1[7]);
+  };
+  auto get = [&](const float4* slot) {
+    const float4 p = slot[lane], q = slot[32 + lane], r = slot[64 + lane], t = slot[96 + lane];
+    v1[0] = p.x; v1[1] = p.y; v1[2] = p.z; v1[3] = p.w;
+    v1[4] = q.x; v1[5] = q.y; v1[6] = q.z; v1[7] = q.w;
+    acc1[0] = r.x; acc1[1] = r.y; acc1[2] = r.z; acc1[3] = r.w;
+    acc1[4] = t.x; acc1[5] = t.y; acc1[6] = t.z; acc1[7] = t.w;
+  };
+
+  int base = 0;  // (-2 k) mod R
+  auto load_segment = [&](int k) {
+    float* dst = rows + (k & 1) * 2 * 32 * kBPitch;
+    load_rows(dst, a.f0, kBT * k * S);
+    load_rows(dst + 32 * kBPitch, a.f1, kBT * k * S - a.min_disp);
+  };
+  load_segment(0);
+  cp_async_commit();
+  for (int k = 0; k < nseg; ++k) {
+    const int s = k * S + w;
+    const int x0 = kBT * s;
+    const bool active = s < nstrips;
+    const bool last = s + 1 == nstrips;  // no strip to the right: blocks end here
+    float v0[kBT], acc0[kBT];
+    // the gradients e = 8 tau .. 8 tau + 7 of the strip's pixels ([x][e];
+    // zeros past the row and the range, and before it in the tile of -1)
+    auto stage = [&](int tau) {
+      if (active && tau <= nb) {
+        float* dst = gt + (tau & (kBGS - 1)) * (kBT * kBT);
+        if constexpr (VEC) {
+          const int x = x0 + (lane >> 1), e = kBT * tau + 4 * (lane & 1);
+          const bool ok = x < a.W && e < a.D && tau >= 0;
+          if (lane < 16) cp_async_or_zero<16>(dst + 4 * lane, ok ? grow + static_cast<int64_t>(x) * a.Dg + e : grow, ok);
+        } else {
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int x = x0 + (lane >> 3) + 4 * h, e = kBT * tau + (lane & 7);
+            const bool ok = x < a.W && e < a.D && tau >= 0;
+            cp_async_or_zero<4>(dst + 32 * h + lane, ok ? grow + static_cast<int64_t>(x) * a.Dg + e : grow, ok);
+          }
+        }
+      }
+      cp_async_commit();
+    };
+    float* seg0 = rows + (k & 1) * 2 * 32 * kBPitch;  // f0, then df0
+    float* seg1 = seg0 + 32 * kBPitch;                // f1, then df1
+    cp_async_wait<0>();
+    __syncthreads();  // the segment's rows have landed; the last one's results are stored
+    if (active) {
+      const float4* p0 = reinterpret_cast<const float4*>(seg0 + lane * kBPitch + kBT * w);
+      const float4* p1 = reinterpret_cast<const float4*>(seg1 + lane * kBPitch + kBT * w);
+      const float4 a0 = p0[0], a1 = p0[1], b0 = p1[0], b1 = p1[1];
+      const float r0[kBT] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+      const float r1[kBT] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+#pragma unroll
+      for (int i = 0; i < kBT; ++i) {
+        const int x = x0 + i, xm = x0 + i - a.min_disp;
+        const bool ok = cok && x < a.W, okm = cok && xm >= 0 && xm < a.W;
+        v0[i] = ok ? r0[i] : qnan;
+        acc0[i] = (ok && a.accum) ? df0r[x] : 0.0f;
+        v1[i] = okm ? r1[i] : qnan;
+        acc1[i] = (okm && a.accum) ? df1r[xm] : 0.0f;
+      }
+    }
+    if (k + 1 < nseg) load_segment(k + 1);
+#pragma unroll
+    for (int t = -1; t < kBGS - 2; ++t) stage(t);
+    for (int tau = 0; tau < nb; ++tau) {
+      if (active && tau > 0) {
+        if (w > 0) {
+          get(xfer + ((tau & 1) * S + w) * 128);
+        } else if (k == 0) {
+          fresh_block(-tau);
+        } else {
+          int slot = base + 2 + tau - 1;  // left segment k - 1 after its step tau - 1
+          slot -= (slot >= R) ? R : 0;
+          get(ring + (slot >= R ? slot - R : slot) * 128);
+        }
+      }
+      cp_async_wait<kBGS - 3>();  // this step's tile has landed
+      __syncwarp();
+      if (active) {
+        // e = 8 tau + ix - iu: for a pixel ix the tiles of tau - 1 and tau
+        // hold its gradients at offsets ix + 1 .. 7 and 0 .. ix
+        const float4* gl = reinterpret_cast<const float4*>(gt + ((tau - 1) & (kBGS - 1)) * (kBT * kBT));
+        const float4* gh = reinterpret_cast<const float4*>(gt + (tau & (kBGS - 1)) * (kBT * kBT));
+#pragma unroll
+        for (int ix = 0; ix < kBT; ++ix) {
+          float gv[2 * kBT];  // gradients e = 8 tau - 8 + q
+          auto quad = [&](int q, const float4 v) {
+            gv[q] = v.x;
+            gv[q + 1] = v.y;
+            gv[q + 2] = v.z;
+            gv[q + 3] = v.w;
+          };
+          if (ix < 3) quad(0, gl[2 * ix]);
+          if (ix < 7) quad(4, gl[2 * ix + 1]);
+          quad(8, gh[2 * ix]);
+          if (ix > 3) quad(12, gh[2 * ix + 1]);
+#pragma unroll
+          for (int iu = kBT - 1; iu >= 0; --iu) sad_pair(v0[ix], v1[iu], gv[kBT + ix - iu], acc0[ix], acc1[iu]);
+        }
+        if (tau == nb - 1) {
+          // (every strip's: stored along the row below)
+          float4* o = reinterpret_cast<float4*>(seg1 + lane * kBPitch + kBT * w);
+          o[0] = make_float4(acc1[0], acc1[1], acc1[2], acc1[3]);
+          o[1] = make_float4(acc1[4], acc1[5], acc1[6], acc1[7]);
+        } else if (last) {
+          store_block(s - tau);
+        } else if (w + 1 < S) {
+          put(xfer + (((tau + 1) & 1) * S + w + 1) * 128);
+        } else {
+          int slot = base + tau;
+          slot -= (slot >= R) ? R : 0;
+          put(ring + slot * 128);
+        }
+      }
+      __syncthreads();
+      stage(tau + kBGS - 2);  // over the tile of tau - 2 (every lane is past it)
+    }
+    if (active) {
+      float4* o = reinterpret_cast<float4*>(seg0 + lane * kBPitch + kBT * w);
+      o[0] = make_float4(acc0[0], acc0[1], acc0[2], acc0[3]);
+      o[1] = make_float4(acc0[4], acc0[5], acc0[6], acc0[7]);
+    }
+    __syncthreads();
+    const int cols = kBT * min(S, nstrips - k * S);
+    store_rows(seg0, a.df0, kBT * k * S, cols);
+    store_rows(seg1, a.df1, kBT * (k * S - (nb - 1)) - a.min_disp, cols);
+    base -= 2;
+    base += (base < 0) ? R : 0;
+  }
+}
+
+constexpr int kGX = 32;            // pixels per block (backward)
+constexpr int kGPX = 4;            // pixels per thread
+constexpr int kGCH = 32;           // channels per block: lane = channel
+constexpr int kGDC = 32;           // disparities per staged chunk
+constexpr int kGFS = kGX + kGDC - 1;  // staged feature row (odd: lanes' rows fall in distinct banks)
 
 // One term of the reference's sums: acc += (diff/|diff|) * g when |diff| >
 // 1e-15 (df0), acc -= ... (df1).  diff/|diff| is exactly +-1, so the update
@@ -226,6 +495,8 @@ __device__ __forceinline__ void sad_term(float& acc, float diff, float g) {
   if (fabsf(diff) > 1e-15f) acc = __fadd_rn(acc, t);
 }
 
+// Both gradients gathered per pixel, for problems with too few rows for the
+// strips below to fill the SMs (sad_bwd_gather).
 // grid (ceil(W/32), H, B*ceil(C/32)); block 256 = 8 warps.  Warp w owns
 // pixels x0 + 4w .. +3, lane the channel; both sums run over d ascending
 // (the reference's order), chunk by chunk of 32 disparities staged in
@@ -236,28 +507,29 @@ __device__ __forceinline__ void sad_term(float& acc, float diff, float g) {
 // is, which is never -0).  Each thread slides a 4-value window over the
 // staged rows, so a disparity costs it one new value per row and one
 // broadcast 16-byte load per gradient table.
-__global__ void __launch_bounds__(256, 3) sad_backward_kernel(SadBwdArgs a) {
+__global__ void __launch_bounds__(256, 3) sad_backward_gather_kernel(SadBwdArgs a) {
   // two buffers: chunk ci + 1 lands (cp.async) while chunk ci is summed
-  __shared__ float f1s[2][kBCH * kBFS];   // f1[c, x0 - d0 - 31 + k]
-  __shared__ float f0s[2][kBCH * kBFS];   // f0[c, x0 + d0 + k]
-  __shared__ __align__(16) float gA[2][kBDC * kBX];  // g[y, x0 + x, d0 + dd]
-  __shared__ __align__(16) float gD[2][kBDC * kBX];  // g[y, x0 + x + d0 + dd, d0 + dd]
-  const int ncb = (a.C + kBCH - 1) / kBCH;
+  __shared__ float f1s[2][kGCH * kGFS];   // f1[c, x0 - d0 - 31 + k]
+  __shared__ float f0s[2][kGCH * kGFS];   // f0[c, x0 + d0 + k]
+  __shared__ __align__(16) float gA[2][kGDC * kGX];  // g[y, x0 + x, d0 + dd]
+  __shared__ __align__(16) float gD[2][kGDC * kGX];  // g[y, x0 + x + d0 + dd, d0 + dd]
+  const int ncb = (a.C + kGCH - 1) / kGCH;
   const int n = blockIdx.z / ncb;
-  const int c0 = (blockIdx.z % ncb) * kBCH;
+  const int c0 = (blockIdx.z % ncb) * kGCH;
   const int y = blockIdx.y;
-  const int x0 = blockIdx.x * kBX;
+  const int x0 = blockIdx.x * kGX;
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const int c = c0 + lane;
   const int64_t HW = static_cast<int64_t>(a.H) * a.W;
+  const int max_disp = a.min_disp + a.D - 1;
   const float* grow = a.g + ((static_cast<int64_t>(n) * a.H + y) * a.W) * a.D;
   const float* f0b = a.f0 + (static_cast<int64_t>(n) * a.C + c0) * HW + static_cast<int64_t>(y) * a.W;
   const float* f1b = a.f1 + (static_cast<int64_t>(n) * a.C + c0) * HW + static_cast<int64_t>(y) * a.W;
   const float qnan = __int_as_float(0x7fffffff);
   // the thread's own pixels: f0[c, x] (df0) and f1[c, x] (df1)
-  float a0[kBPX], b0[kBPX], acc0[kBPX], acc1[kBPX];
+  float a0[kGPX], b0[kGPX], acc0[kGPX], acc1[kGPX];
 #pragma unroll
-  for (int i = 0; i < kBPX; ++i) {
+  for (int i = 0; i < kGPX; ++i) {
     const int x = x0 + 4 * w + i;
     const bool ok = c < a.C && x < a.W;
     a0[i] = ok ? __ldg(f0b + lane * HW + x) : 0.0f;
@@ -267,23 +539,23 @@ __global__ void __launch_bounds__(256, 3) sad_backward_kernel(SadBwdArgs a) {
   }
   // stage chunk ci into buffer ci & 1: cp.async for what lies inside the
   // image and the disparity range, plain stores of the fill values
-  const int nchunk = (a.max_disp - a.min_disp) / kBDC + 1;
+  const int nchunk = (max_disp - a.min_disp) / kGDC + 1;
   auto stage = [&](int ci) {
     const int b = ci & 1;
-    const int d0 = a.min_disp + ci * kBDC;
+    const int d0 = a.min_disp + ci * kGDC;
     const int i0 = d0 - a.min_disp;
-    const int nd = min(kBDC, a.max_disp - d0 + 1);
-    for (int e = tid; e < kBCH * kBFS; e += 256) {
-      const int cc = e / kBFS, k = e - cc * kBFS;
+    const int nd = min(kGDC, max_disp - d0 + 1);
+    for (int e = tid; e < kGCH * kGFS; e += 256) {
+      const int cc = e / kGFS, k = e - cc * kGFS;
       const bool cok = c0 + cc < a.C;
-      const int xa = x0 - d0 - (kBDC - 1) + k, xb = x0 + d0 + k;
+      const int xa = x0 - d0 - (kGDC - 1) + k, xb = x0 + d0 + k;
       if (cok && xa >= 0 && xa < a.W) cp_async4(&f1s[b][e], f1b + cc * HW + xa);
       else f1s[b][e] = qnan;
       if (cok && xb >= 0 && xb < a.W) cp_async4(&f0s[b][e], f0b + cc * HW + xb);
       else f0s[b][e] = qnan;
     }
-    for (int e = tid; e < kBDC * kBX; e += 256) {
-      const int dd = e / kBX, x = e - dd * kBX;
+    for (int e = tid; e < kGDC * kGX; e += 256) {
+      const int dd = e / kGX, x = e - dd * kGX;
       const int xa = x0 + x, xd = x0 + x + d0 + dd;
       if (dd < nd && xa < a.W) cp_async4(&gA[b][e], grow + static_cast<int64_t>(xa) * a.D + i0 + dd);
       else gA[b][e] = 0.0f;
@@ -302,30 +574,30 @@ __global__ void __launch_bounds__(256, 3) sad_backward_kernel(SadBwdArgs a) {
       cp_async_wait<0>();
     }
     __syncthreads();
-    const float* F1 = f1s[b] + lane * kBFS + 4 * w + (kBDC - 1);  // F1[i - dd] = f1[c, x0 + 4w + i - (d0 + dd)]
-    const float* F0 = f0s[b] + lane * kBFS + 4 * w;               // F0[i + dd] = f0[c, x0 + 4w + i + (d0 + dd)]
-    float v1[kBPX], v0[kBPX];
+    const float* F1 = f1s[b] + lane * kGFS + 4 * w + (kGDC - 1);  // F1[i - dd] = f1[c, x0 + 4w + i - (d0 + dd)]
+    const float* F0 = f0s[b] + lane * kGFS + 4 * w;               // F0[i + dd] = f0[c, x0 + 4w + i + (d0 + dd)]
+    float v1[kGPX], v0[kGPX];
 #pragma unroll
-    for (int i = 0; i < kBPX; ++i) {
+    for (int i = 0; i < kGPX; ++i) {
       v1[i] = F1[i];
       v0[i] = F0[i];
     }
 #pragma unroll
-    for (int dd = 0; dd < kBDC; ++dd) {
+    for (int dd = 0; dd < kGDC; ++dd) {
       if (dd > 0) {
 #pragma unroll
-        for (int i = kBPX - 1; i > 0; --i) v1[i] = v1[i - 1];
+        for (int i = kGPX - 1; i > 0; --i) v1[i] = v1[i - 1];
         v1[0] = F1[-dd];
 #pragma unroll
-        for (int i = 0; i < kBPX - 1; ++i) v0[i] = v0[i + 1];
-        v0[kBPX - 1] = F0[kBPX - 1 + dd];
+        for (int i = 0; i < kGPX - 1; ++i) v0[i] = v0[i + 1];
+        v0[kGPX - 1] = F0[kGPX - 1 + dd];
       }
-      const float4 ga = *reinterpret_cast<const float4*>(gA[b] + dd * kBX + 4 * w);
-      const float4 gd = *reinterpret_cast<const float4*>(gD[b] + dd * kBX + 4 * w);
+      const float4 ga = *reinterpret_cast<const float4*>(gA[b] + dd * kGX + 4 * w);
+      const float4 gd = *reinterpret_cast<const float4*>(gD[b] + dd * kGX + 4 * w);
       const float gav[4] = {ga.x, ga.y, ga.z, ga.w};
       const float gdv[4] = {gd.x, gd.y, gd.z, gd.w};
 #pragma unroll
-      for (int i = 0; i < kBPX; ++i) {
+      for (int i = 0; i < kGPX; ++i) {
         sad_term<false>(acc0[i], __fsub_rn(a0[i], v1[i]), gav[i]);
         sad_term<true>(acc1[i], __fsub_rn(v0[i], b0[i]), gdv[i]);
       }
@@ -334,13 +606,28 @@ __global__ void __launch_bounds__(256, 3) sad_backward_kernel(SadBwdArgs a) {
   }
   if (c >= a.C || c >= a.channel_limit) return;
 #pragma unroll
-  for (int i = 0; i < kBPX; ++i) {
+  for (int i = 0; i < kGPX; ++i) {
     const int x = x0 + 4 * w + i;
     if (x >= a.W) continue;
     const int64_t o = (static_cast<int64_t>(n) * a.C + c) * HW + static_cast<int64_t>(y) * a.W + x;
     a.df0[o] = acc0[i];
     a.df1[o] = acc1[i];
   }
+}
+
+// Whether the gather form is the faster one: the strips run one block per
+// image row and 32 channels, an SM at a time, 1.25 us per step of 64 pairs a
+// warp; the gather form 3 blocks of 32 pixels per SM, 0.28 us per disparity.
+// Strips against gather, C = 32, W = 1240, D = 192 (10 segments of 25 steps):
+// 10 rows 0.32 / 0.06 ms, 60 rows 0.32 / 0.30, 94 rows 0.32 / 0.45, 188 rows
+// 0.63 / 0.90; 4x64x100, D = 64: 36 / 63 us; C = 48, 376x333, D = 50: 0.18 /
+// 0.29 ms.
+bool sad_bwd_gather(int B, int C, int H, int W, int D) {
+  const int64_t rows = static_cast<int64_t>(B) * H * ((C + 31) / 32), sms = sm_count();
+  const int strips = (W + kBT - 1) / kBT, nseg = (strips + kBWarps - 1) / kBWarps;
+  const double t_strips = 1.25 * ((rows + sms - 1) / sms) * nseg * sad_bwd_blocks(D);
+  const double t_gather = 0.28 * D * std::max(1.0, static_cast<double>(rows * ((W + kGX - 1) / kGX)) / (3 * sms) + 0.25);
+  return t_gather < t_strips;
 }
 
 }  // namespace
@@ -402,14 +689,45 @@ extern "C" int bpl_sad_backward(const float* f0, const float* f1, const float* i
   BPL_REQUIRE(f0 && f1 && in_grad && df0 && df1, "sad_backward: null pointer");
   BPL_REQUIRE(B >= 1 && C >= 1 && H >= 1 && W >= 1 && max_disp >= min_disp, "sad_backward: bad shape");
   const int D = max_disp - min_disp + 1;
-  SadBwdArgs a{f0, f1, in_grad, df0, df1, B, C, H, W, D, min_disp, max_disp, C};
+  BPL_REQUIRE(static_cast<int64_t>(B) * ((C + 31) / 32) <= 65535 && H <= 65535 &&
+                  static_cast<int64_t>(H) * ((C + 31) / 32) < (1ll << 31),
+              "sad_backward: grid too large");
+  SadBwdArgs a{f0, f1, in_grad, df0, df1, B, C, H, W, 0, 0, D, 0, 0, 0, C};
   // the reference launch covers only 4*ceil(D/4) channels (stereo_sad_kernel.cu:152-157)
   if (reference_channel_limit) a.channel_limit = std::min(C, 4 * ((D + 3) / 4));
-  BPL_CUDA_TRY(cudaMemsetAsync(df0, 0, sizeof(float) * B * C * H * W, as_stream(stream)), "sad_backward: memset");
-  BPL_CUDA_TRY(cudaMemsetAsync(df1, 0, sizeof(float) * B * C * H * W, as_stream(stream)), "sad_backward: memset");
-  BPL_REQUIRE(static_cast<int64_t>(B) * ((C + kBCH - 1) / kBCH) <= 65535 && H <= 65535, "sad_backward: grid too large");
-  dim3 grid((W + kBX - 1) / kBX, H, B * ((C + kBCH - 1) / kBCH));
-  sad_backward_kernel<<<grid, 256, 0, as_stream(stream)>>>(a);
-  BPL_CUDA_TRY(cudaGetLastError(), "sad_backward launch");
+  // what the kernel does not write: channels past the limit, and f1 columns
+  // that no disparity reaches (none when the range starts at 0)
+  if (a.channel_limit < C)
+    BPL_CUDA_TRY(cudaMemsetAsync(df0, 0, sizeof(float) * B * C * H * W, as_stream(stream)), "sad_backward: memset");
+  if (a.channel_limit < C || min_disp != 0)
+    BPL_CUDA_TRY(cudaMemsetAsync(df1, 0, sizeof(float) * B * C * H * W, as_stream(stream)), "sad_backward: memset");
+  if (sad_bwd_gather(B, C, H, W, D)) {
+    a.D = D;
+    a.min_disp = min_disp;
+    dim3 grid((W + kGX - 1) / kGX, H, B * ((C + kGCH - 1) / kGCH));
+    sad_backward_gather_kernel<<<grid, 256, 0, as_stream(stream)>>>(a);
+    BPL_CUDA_TRY(cudaGetLastError(), "sad_backward launch");
+    return BPL_OK;
+  }
+  const int strips = std::min(kBWarps, (W + kBT - 1) / kBT);
+  // wide ranges in launches of kBMaxD disparities (their blocks in flight
+  // fill the shared memory), the sums carried on in order
+  for (int g0 = 0; g0 < D; g0 += kBMaxD) {
+    a.D = std::min(kBMaxD, D - g0);
+    a.min_disp = min_disp + g0;
+    a.g0 = g0;
+    a.accum = g0 > 0 ? 1 : 0;
+    a.nb = sad_bwd_blocks(a.D);
+    const size_t smem = sad_bwd_smem_bytes(strips, a.nb);
+    if (static_cast<int>(smem) > max_smem_optin())
+      return set_error(BPL_ERR_UNSUPPORTED, "sad_backward: shared memory %zu exceeds device limit", smem);
+    const bool vec = reinterpret_cast<uintptr_t>(in_grad) % 16 == 0 && D % 4 == 0;
+    auto kern = vec ? sad_backward_kernel<true> : sad_backward_kernel<false>;
+    BPL_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)),
+                 "cudaFuncSetAttribute");
+    dim3 grid(H * ((C + 31) / 32), B);
+    kern<<<grid, 32 * strips, smem, as_stream(stream)>>>(a);
+    BPL_CUDA_TRY(cudaGetLastError(), "sad_backward launch");
+  }
   return BPL_OK;
 }
