@@ -53,9 +53,6 @@ int lbp_forward_impl(int storage, int variant, const void* cost, const void* jum
   a.eb = edge_batch;
   a.delta = delta;
   a.argmin_kind = argmin_kind;
-  a.am_vec = (reinterpret_cast<uintptr_t>(argmin) | static_cast<uintptr_t>(L)) % 16 == 0  ? 16
-             : (reinterpret_cast<uintptr_t>(argmin) | static_cast<uintptr_t>(L)) % 4 == 0 ? 4
-                                                                                          : 1;
   a.planes2 = planes2;
   a.lrow = align4(L);
   if (storage == 0) {
@@ -73,6 +70,9 @@ int lbp_forward_impl(int storage, int variant, const void* cost, const void* jum
     a.lmat = (variant == BPL_LBP_SEM_PIXEL && L <= kPixelRingMaxL) ? L * a.Lm : 0;
     a.vec4 = 1;
   }
+  const uintptr_t am_at = reinterpret_cast<uintptr_t>(argmin) | static_cast<uintptr_t>(a.Ls);
+  a.am_vec = (am_at % 16 == 0) ? 16 : (am_at % 4 == 0) ? 4 : 1;
+  a.half_align = ((reinterpret_cast<uintptr_t>(cost) | reinterpret_cast<uintptr_t>(messages)) % 16 == 0) ? 1 : 0;
   // shared-memory ring (pixel variant up to kPixelRingMaxL labels): 4 steps
   // in flight, one step per mbarrier group; the other variants, and wider
   // pixel rows, prefetch rows into registers (wider pixel rows read their

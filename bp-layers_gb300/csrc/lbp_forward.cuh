@@ -84,6 +84,7 @@ struct FwdArgs {
   int Ls;     // label stride of cost / messages / argmin rows
   int Lm;     // row stride of the pixel-pairwise matrices (pixel variant)
   int argmin_kind;
+  int half_align;  // half storage: cost and messages start on 16-byte boundaries
   int am_vec;  // uint8 argmin rows start on multiples of this many bytes and are multiples of it long (16, 4 or 1)
   int phase;  // 0: RIGHT+LEFT over rows, 1: DOWN+UP over columns
   int nchains;

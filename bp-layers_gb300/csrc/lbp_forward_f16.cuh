@@ -1,8 +1,8 @@
 // Min-sum LBP forward with FP16 storage, stereo pairwise: the lean step.
 //
-// Same sweeps, scanline ownership and label layout as lbp_forward_kernel
-// (one warp walks one scanline of one sweep, label = lane + 32k, the chain
-// message stays in registers), but the step is built for FP16 storage, which
+// Same sweeps and scanline ownership as lbp_forward_kernel (one warp walks one
+// scanline of one sweep, the chain message stays in registers; labels go to
+// lanes in pairs), but the step is built for FP16 storage, which
 // has no bitwise target:
 //   * every stored row is the min-sum message minus the minimum of h over
 //     the sender's labels (min-normalisation): no exp, no sum, no log on the
@@ -25,44 +25,81 @@
 // ops/lbp_stereo/src/lbp_min_sum_kernel.cu:55-164.
 #pragma once
 
+
 #include <type_traits>
-#include <utility>
 
 #include "lbp_forward.cuh"
 
 namespace bpl {
 
-// compile-time loop: f(integral_constant<int, 0>), ..., f(integral_constant<int, N-1>)
-template <typename F, int... I>
-__device__ __forceinline__ void static_for_impl(F& f, std::integer_sequence<int, I...>) {
-  (f(std::integral_constant<int, I>{}), ...);
-}
-template <int N, typename F>
-__device__ __forceinline__ void static_for(F&& f) {
-  static_for_impl(f, std::make_integer_sequence<int, N>{});
+// steps of rows in the shared-memory ring (a power of two; 0: no ring)
+template <int OCC>
+constexpr int f16_depth = (OCC > 1) ? 0 : 8;
+// steps ahead of the L2 prefetch (no ring)
+constexpr int kF16Ahead = 8;
+// floats of a warp's shared memory: h row, ring, two tap tiles
+__host__ __device__ inline int f16_warp_floats(int NP, int depth, int Lv) {
+  return align4(64 * NP + 2 * kHsPad) + depth * 3 * 32 * NP + 2 * tap_tile_floats(Lv, true);
 }
 
 template <int OCC>
 constexpr int f16_block_warps() { return (OCC > 1) ? 1 : 4; }
 
-// PF: prefetch depth (steps whose rows are in flight).  The lean step is
-// short, so one step ahead does not cover a DRAM load (ncu: long-scoreboard
-// stalls led the one-ahead version); the 4-warp, latency-bound launch keeps
-// three steps in flight, the high-occupancy launch one (its other warps hide
-// the latency, and it has no registers to spare).
-template <int K, int OCC, bool SCALE, int PF>
+// The window of a sender as the usual step reads it: {w, L2, f(t-1), f(t+1)}
+// and {f(t), 1 where the beating offsets are exactly |jd| <= 1 (see
+// classify_taps), else 0}, in the place of the float kernel's lean records.
+__device__ __forceinline__ void store_f16_record(const FwdArgs& a, float* tile, int lane) {
+  const int c0 = a.Lv / 2;
+  const int code = __float_as_int(tile[(a.Lv + 2) * 33 + lane]) & 0xff;
+  float* rec = tile + lean_off(a.Lv);
+  reinterpret_cast<float4*>(rec)[lane] =
+      make_float4(tile[a.Lv * 33 + lane], tile[(a.Lv - 1) * 33 + lane], tile[min(a.Lv - 1, c0 + 1) * 33 + lane],
+                  tile[max(1, c0 - 1) * 33 + lane]);
+  reinterpret_cast<float2*>(rec + 128)[lane] = make_float2(tile[c0 * 33 + lane], code == 3 ? 1.0f : 0.0f);
+}
+
+// Labels in pairs: lane l holds labels 64 p + 2 l and the next one, p < NP =
+// ceil(L/64), as half2 in memory (no reduction here depends on an order of
+// labels, unlike the float kernel's sum).  A pair costs one 4-byte access per
+// row instead of two of 2 bytes, one 8-byte store to the h row and two reads
+// of its neighbours instead of four.
+// The rows of the next steps (cost and the two cross-direction messages): with
+// few warps per SM (4-warp blocks) through a shared-memory ring by 16-byte
+// cp.async, a few lanes per row, 8 steps in flight: the step is shorter than a
+// DRAM or L2 access, and loads into registers two or three steps ahead still
+// waited for the newest of them (horizontal launch at 376x1240x128 0.55 ms,
+// 0.41 with the ring).  The one-warp blocks load into registers two steps
+// ahead (slots by the step's parity), the rows in L2 by then (kF16Ahead):
+// vertical launch at 376x1240x192 0.36 ms, 0.44 with one step ahead, 0.47
+// with a ring; at 376x1240x128 0.22 ms, 0.28 without the L2 prefetch.
+// AM: an argmin is stored.  PH: the phase (h is summed in another order).
+//
+// What bounds it: along rows the step's latency and its instructions (about
+// 180 without an argmin at 128 labels, 320 with one at 192, three cycles
+// each); down columns DRAM (1.1 GB read and 0.5 written per launch at
+// 376x1240x192 in 0.36 ms, 70 % of the copy rate).  Per pass at 376x1240x192
+// with argmin 1.43 -> 1.00 ms (rows 0.89 -> 0.64, columns 0.54 -> 0.36), at
+// 376x1240x128 without 1.08 -> 0.64 ms.
+template <int NP, int OCC, bool AM, int PH>
 __global__ void __launch_bounds__(32 * f16_block_warps<OCC>(), OCC) lbp_forward_f16_kernel(FwdArgs a) {
+  constexpr int K = 2 * NP;
+  constexpr int DEPTH = f16_depth<OCC>;
+  constexpr bool kRing = DEPTH > 0;
+  constexpr int SLOTS = kRing ? 1 : 2;
+  using Slot0 = std::integral_constant<int, 0>;
+  using Slot1 = std::integral_constant<int, SLOTS - 1>;
   extern __shared__ __align__(16) float smem[];
   const int lane = threadIdx.x & 31;
   const int wib = threadIdx.x >> 5;
   const int chain_id = blockIdx.x * (blockDim.x >> 5) + wib;
   if (chain_id >= a.nchains) return;
 
-  // per warp: h row (32K + 2 pads) and the two-block tap tile
-  const int tile_stride = tap_tile_rows(a.Lv) * 33;
-  float* base = smem + static_cast<int64_t>(wib) * (align4(32 * K + 2 * kHsPad) + 2 * tile_stride);
+  // per warp: h row (64 NP + 2 pads), the rows' ring, the two-block tap tile
+  const int tile_stride = tap_tile_floats(a.Lv, true);
+  float* base = smem + static_cast<int64_t>(wib) * f16_warp_floats(NP, DEPTH, a.Lv);
   float* hs = base + kHsPad;
-  float* taps = base + align4(32 * K + 2 * kHsPad);
+  __half* ring = reinterpret_cast<__half*>(base + align4(32 * K + 2 * kHsPad));  // [DEPTH][3][64 NP]
+  float* taps = base + align4(32 * K + 2 * kHsPad) + DEPTH * 3 * 32 * NP;
   if (lane < kHsPad) {
     hs[-1 - lane] = __int_as_float(0x7f800000);
     hs[32 * K + lane] = __int_as_float(0x7f800000);
@@ -76,7 +113,7 @@ __global__ void __launch_bounds__(32 * f16_block_warps<OCC>(), OCC) lbp_forward_
   int len;
   {
     const int r = chain_id >> 1;
-    if (a.phase == 0) {
+    if (PH == 0) {
       c.dir = (chain_id & 1) ? LEFT : RIGHT;
       c.n = r / a.H;
       const int y = r % a.H;
@@ -95,93 +132,269 @@ __global__ void __launch_bounds__(32 * f16_block_warps<OCC>(), OCC) lbp_forward_
   const int nsteps = len - 1;
   if (nsteps <= 0) return;
   const int od = c.dir ^ 1;
-  const int sa = (a.phase == 0) ? UP : RIGHT;
-  const int sb = (a.phase == 0) ? DOWN : LEFT;
-  const __half* cost = static_cast<const __half*>(a.cost) + static_cast<int64_t>(c.n) * HWL;
-  const __half* slot_a = static_cast<const __half*>(a.msgs) + (static_cast<int64_t>(c.n) * 4 + sa) * HWL;
-  const __half* slot_b = static_cast<const __half*>(a.msgs) + (static_cast<int64_t>(c.n) * 4 + sb) * HWL;
+  const int sa = (PH == 0) ? UP : RIGHT;
+  const int sb = (PH == 0) ? DOWN : LEFT;
   c.out_off = (static_cast<int64_t>(c.n) * 4 + od) * HWL;
-  __half* slot_out = static_cast<__half*>(a.msgs) + c.out_off;
   c.t0 = 0;
-  float* scale_out = SCALE ? a.scale + (static_cast<int64_t>(c.n) * 4 + od) * HW : nullptr;
-  // only the last slot can hold labels >= L (K = ceil(L/32))
-  auto lvalid = [&](int kk) -> bool { return kk < K - 1 || lane + 32 * kk < L; };
-
-  // the next step's cost and cross-direction messages, one step ahead
-  __half pcst[PF][K], pva[PF][K], pvb[PF][K];
-  auto prefetch = [&](auto SL, int i) {
-    constexpr int sl = decltype(SL)::value;
-    const int64_t po = static_cast<int64_t>(c.pin0 + i * c.dpin) * Ls;
+  float* scale_out = a.scale ? a.scale + (static_cast<int64_t>(c.n) * 4 + od) * HW : nullptr;
+  // label of slot kk; the last pair alone can hold labels >= L
+  auto lab = [&](int kk) -> int { return 64 * (kk >> 1) + 2 * lane + (kk & 1); };
+  auto lvalid = [&](int kk) -> bool { return kk < K - 2 || lab(kk) < L; };
+  const int64_t pstep = static_cast<int64_t>(c.dpin) * Ls;
+  __half* slot_out = static_cast<__half*>(a.msgs) + c.out_off;
+  const int64_t p0 = static_cast<int64_t>(c.pin0) * Ls;
+  const __half* rows[3] = {static_cast<const __half*>(a.cost) + static_cast<int64_t>(c.n) * HWL + p0,
+                           static_cast<const __half*>(a.msgs) + (static_cast<int64_t>(c.n) * 4 + sa) * HWL + p0,
+                           static_cast<const __half*>(a.msgs) + (static_cast<int64_t>(c.n) * 4 + sb) * HWL + p0};
+  const bool aligned = a.half_align != 0;
+  // ring: the three rows of a step as 16-byte chunks, lane + 32 q the chunk
+  // (row, place) of copy q; one group per step (empty past the end)
+  constexpr int NC = (24 * NP + 31) / 32;
+  const __half* src[NC];
+  bool mine[NC];
 #pragma unroll
-    for (int kk = 0; kk < K; ++kk) {
-      const int64_t o = po + (lvalid(kk) ? lane + 32 * kk : 0);
-      pcst[sl][kk] = __ldg(cost + o);
-      pva[sl][kk] = __ldg(slot_a + o);
-      pvb[sl][kk] = __ldg(slot_b + o);
+  for (int q = 0; q < NC; ++q) {
+    const int e = lane + 32 * q, r = e / (8 * NP), at = e % (8 * NP);
+    mine[q] = r < 3 && 8 * at < Ls;
+    src[q] = (r == 1 ? rows[1] : r == 2 ? rows[2] : rows[0]) + 8 * at;
+  }
+  // no ring: the next step's pairs (those wholly past L stay zero: masked),
+  // and this lane's line of the rows kF16Ahead steps further on
+  unsigned nxt[SLOTS][3][NP];
+  const int prow = lane / (NP + 1), pline = lane % (NP + 1);
+  const char* ppf = reinterpret_cast<const char*>((prow == 1 ? rows[1] : prow == 2 ? rows[2] : rows[0]) +
+                                                  min(kF16Ahead, nsteps - 1) * pstep) +
+                    ((prow < 3 && 64 * pline < L) ? 128 * pline : 0);
+#pragma unroll
+  for (int k = 0; k < SLOTS; ++k) nxt[k][0][NP - 1] = nxt[k][1][NP - 1] = nxt[k][2][NP - 1] = 0u;
+#pragma unroll
+  for (int r = 0; r < 3; ++r) rows[r] += 2 * lane;
+  // brings in step i's rows (in order of i), into register slot SL
+  auto issue = [&](auto SL, int i) {
+    constexpr int sl = decltype(SL)::value;
+    if constexpr (kRing) {
+      if (i < nsteps) {
+        __half* dst = ring + (i & (DEPTH - 1)) * (3 * 64 * NP);
+        if (__builtin_expect(aligned, 1)) {
+#pragma unroll
+          for (int q = 0; q < NC; ++q)
+            if (mine[q]) cp_async16(dst + 8 * (lane + 32 * q), src[q]);
+        } else {
+          // (tensors that do not start on a 16-byte boundary)
+          for (int q = 0; q < NC; ++q)
+            if (mine[q])
+              for (int k = 0; k < 8; ++k) dst[8 * (lane + 32 * q) + k] = src[q][k];
+        }
+#pragma unroll
+        for (int q = 0; q < NC; ++q) src[q] += pstep;
+      }
+      cp_async_commit();
+    } else {
+      if (i < nsteps) {
+        if (__builtin_expect(aligned, 1)) {
+#pragma unroll
+          for (int p = 0; p < NP; ++p)
+            if (lvalid(2 * p)) {
+#pragma unroll
+              for (int r = 0; r < 3; ++r) nxt[sl][r][p] = __ldg(reinterpret_cast<const unsigned*>(rows[r] + 64 * p));
+            }
+        } else {
+          for (int p = 0; p < NP; ++p)
+            if (lvalid(2 * p)) {
+#pragma unroll
+              for (int r = 0; r < 3; ++r) {
+                const unsigned short* u = reinterpret_cast<const unsigned short*>(rows[r] + 64 * p);
+                nxt[sl][r][p] = __ldg(u) | (static_cast<unsigned>(__ldg(u + 1)) << 16);
+              }
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < 3; ++r) rows[r] += pstep;
+      }
+      prefetch_l2(ppf);
+      ppf += (i + kF16Ahead < nsteps) ? pstep * 2 : 0;
     }
   };
-  static_for<PF>([&](auto SL) {
-    constexpr int s = decltype(SL)::value;
-    if (s < nsteps) prefetch(SL, s);
-  });
+  // pair p of row r of step i
+  auto pair = [&](auto SL, int i, int r, int p) -> float2 {
+    constexpr int sl = decltype(SL)::value;
+    __half2 v;
+    if constexpr (kRing)
+      v = *reinterpret_cast<const __half2*>(ring + ((i & (DEPTH - 1)) * 3 + r) * (64 * NP) + 64 * p + 2 * lane);
+    else
+      v = *reinterpret_cast<const __half2*>(&nxt[sl][r][p]);
+    return __half22float2(v);
+  };
 
   float chain[K];
   {
     const __half* src = slot_out + static_cast<int64_t>(c.pin0) * Ls;
 #pragma unroll
-    for (int kk = 0; kk < K; ++kk) chain[kk] = lvalid(kk) ? __half2float(src[lane + 32 * kk]) : 0.0f;
+    for (int kk = 0; kk < K; ++kk) chain[kk] = lvalid(kk) ? __half2float(src[lab(kk)]) : 0.0f;
   }
 
-  TapRegs tr;
-  load_taps(a, c, 0, lane, nsteps, tr, true);
-  store_taps(a, taps, lane, tr, true);
-  if (nsteps > 32) load_taps(a, c, 1, lane, nsteps, tr, true);
+  stage_taps(a, c, 0, lane, nsteps, taps);
+  cp_async_wait<0>();
+  classify_taps(a, taps, lane);
+  store_f16_record(a, taps, lane);
+  if (nsteps > 32) stage_taps(a, c, 1, lane, nsteps, taps + tile_stride);
+  if constexpr (kRing) {
+    for (int k = 0; k < DEPTH - 1; ++k) issue(Slot0{}, k);
+    cp_async_wait<DEPTH - 2>();  // step 0 has landed
+  } else {
+    issue(Slot0{}, 0);
+    issue(Slot1{}, 1);
+  }
   __syncwarp();
 
   const int delta = a.delta;
-  const bool store_am = a.argmin_kind != BPL_ARGMIN_NONE;
   const float kInf = __int_as_float(0x7f800000);
   const int c0 = a.Lv / 2;
-  auto step = [&](auto SL, const int i) {
-    constexpr int sl = decltype(SL)::value;
-    const int pin = c.pin0 + i * c.dpin;
-    const int j = i & 31;
-    const int b = i >> 5;
-    const float* tile = taps + (b & 1) * tile_stride;
-
-    // h = cost + incoming messages except the chain direction's own slot,
-    // in the reference's order (RIGHT, LEFT, UP, DOWN)
-    float h[K];
-    float pm = kInf;
+  __half* pd = slot_out + static_cast<int64_t>(c.pin0 + c.dpin) * Ls + 2 * lane;
+  uint8_t* pam = static_cast<uint8_t*>(a.argmin) + c.out_off + static_cast<int64_t>(c.pin0 + c.dpin) * Ls + 2 * lane;
+  const bool am_pairs = a.argmin_kind == BPL_ARGMIN_U8 && a.am_vec > 1;
+  float h[K], msg[K], pm = 0.0f;
+  int am[K], argmin_h = 0;
+  int i = 0;
+  // h = cost + incoming messages except the chain direction's own slot, in
+  // the reference's order (RIGHT, LEFT, UP, DOWN), its row in shared memory
+  // and its minimum
+  auto head = [&](auto SL) {
 #pragma unroll
-    for (int kk = 0; kk < K; ++kk) {
-      const float cst = __half2float(pcst[sl][kk]);
-      const float va = __half2float(pva[sl][kk]);
-      const float vb = __half2float(pvb[sl][kk]);
-      const float hv = (a.phase == 0) ? ((cst + chain[kk]) + va) + vb : ((cst + va) + vb) + chain[kk];
-      h[kk] = lvalid(kk) ? hv : kInf;
-      hs[lane + 32 * kk] = h[kk];
-      pm = fminf(pm, h[kk]);
+    for (int p = 0; p < NP; ++p) {
+      const float2 cst = pair(SL, i, 0, p), va = pair(SL, i, 1, p), vb = pair(SL, i, 2, p);
+      h[2 * p] = (PH == 0) ? ((cst.x + chain[2 * p]) + va.x) + vb.x : ((cst.x + va.x) + vb.x) + chain[2 * p];
+      h[2 * p + 1] =
+          (PH == 0) ? ((cst.y + chain[2 * p + 1]) + va.y) + vb.y : ((cst.y + va.y) + vb.y) + chain[2 * p + 1];
+      if (!lvalid(2 * p)) h[2 * p] = kInf;
+      if (!lvalid(2 * p + 1)) h[2 * p + 1] = kInf;
+      *reinterpret_cast<float2*>(hs + 64 * p + 2 * lane) = make_float2(h[2 * p], h[2 * p + 1]);
     }
-    pm = warp_min_redux(pm);
-    int argmin_h = 0;
-    if (store_am) {
+    pm = warp_min_f32(slot_min<K>(h));
+    __syncwarp();  // h of the whole pixel is visible in hs
+    issue(SL, i + (kRing ? DEPTH - 1 : 2));  // (ring: over the rows of step i - 1, which every lane is past)
+    if (AM) {
       int ll = -1;
 #pragma unroll
-      for (int kk = 0; kk < K; ++kk) ll = (h[kk] == pm) ? lane + 32 * kk : ll;
+      for (int kk = 0; kk < K; ++kk) ll = (h[kk] == pm) ? lab(kk) : ll;
       argmin_h = __reduce_max_sync(FULL, ll);
     }
-    __syncwarp();  // h of the whole pixel is visible in hs
-    if (i + PF < nsteps) prefetch(SL, i + PF);
-
+  };
+  // stores the row relative to the minimum of h (the chain carries the
+  // stored, half-rounded value, so it matches memory), its argmin and scale,
+  // and goes to the next step; true at the end of the scanline
+  auto tail = [&]() -> bool {
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+      const __half2 o = __floats2half2_rn(msg[2 * p] - pm, msg[2 * p + 1] - pm);
+      const float2 f = __half22float2(o);
+      chain[2 * p] = f.x;
+      chain[2 * p + 1] = f.y;
+      if (aligned && lvalid(2 * p + 1)) {  // (rows of whole 16 bytes)
+        *reinterpret_cast<__half2*>(pd + 64 * p) = o;
+      } else {
+        if (lvalid(2 * p)) pd[64 * p] = __low2half(o);
+        if (lvalid(2 * p + 1)) pd[64 * p + 1] = __high2half(o);
+      }
+    }
+    if (AM) {
+      if (am_pairs) {
+#pragma unroll
+        for (int p = 0; p < NP; ++p) {
+          if (lvalid(2 * p + 1))
+            *reinterpret_cast<uint16_t*>(pam + 64 * p) = static_cast<uint16_t>(am[2 * p] | (am[2 * p + 1] << 8));
+          else if (lvalid(2 * p)) pam[64 * p] = static_cast<uint8_t>(am[2 * p]);
+        }
+      } else {
+        const int64_t ao = c.out_off + static_cast<int64_t>(c.pin0 + (i + 1) * c.dpin) * Ls;
+#pragma unroll
+        for (int kk = 0; kk < K; ++kk) {
+          if (!lvalid(kk)) continue;
+          if (a.argmin_kind == BPL_ARGMIN_U8) static_cast<uint8_t*>(a.argmin)[ao + lab(kk)] = static_cast<uint8_t>(am[kk]);
+          else if (a.argmin_kind == BPL_ARGMIN_U16) static_cast<uint16_t*>(a.argmin)[ao + lab(kk)] = static_cast<uint16_t>(am[kk]);
+          else static_cast<float*>(a.argmin)[ao + lab(kk)] = static_cast<float>(am[kk]);
+        }
+      }
+      pam += pstep;
+    }
+    if (scale_out != nullptr) {
+      float esum = 0.0f;
+#pragma unroll
+      for (int kk = 0; kk < K; ++kk) esum += lvalid(kk) ? __expf(chain[kk]) : 0.0f;
+      esum = warp_sum(esum);
+      if (lane == 0) scale_out[c.pin0 + (i + 1) * c.dpin] = esum;
+    }
+    pd += pstep;
+    ++i;
+    if constexpr (kRing) cp_async_wait<DEPTH - 2>();  // the next step's rows have landed
+    __syncwarp();                                     // (and hs is rewritten by it)
+    if ((i & 31) == 0 && i < nsteps) {
+      // next tap block
+      const int b = i >> 5;
+      float* next = taps + (b & 1) * tile_stride;
+      // (with a ring: its copies, issued 32 steps ago, are older than the
+      // rows just waited for)
+      if constexpr (!kRing) cp_async_wait<0>();
+      classify_taps(a, next, lane);
+      store_f16_record(a, next, lane);
+      if (32 * (b + 1) < nsteps) stage_taps(a, c, b + 1, lane, nsteps, taps + ((b + 1) & 1) * tile_stride);
+      __syncwarp();
+    }
+    return i == nsteps;
+  };
+  // One step of the usual window (lbp_min_sum_kernel.cu:112-164 with the
+  // terms |jd| <= 1): the candidate L2*w + min h, and the terms that can beat
+  // it.  0: done, 1: the general step has to finish it, 2: end of the
+  // scanline.
+  auto usual = [&](auto SL) -> int {
+    const float* rec = taps + ((i >> 5) & 1) * tile_stride + lean_off(a.Lv);
+    const float4 lt = reinterpret_cast<const float4*>(rec)[i & 31];
+    const float2 l2 = reinterpret_cast<const float2*>(rec + 128)[i & 31];
+    head(SL);
+    if (l2.y == 0.0f || delta >= L) return 1;
+    const float w = lt.x;
+    const float msg_g = __fmaf_rn(lt.y, w, pm);
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+      const float hl = hs[64 * p + 2 * lane - 1], hr = hs[64 * p + 2 * lane + 2];
+      const float x[4] = {hl, h[2 * p], h[2 * p + 1], hr};
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const int kk = 2 * p + q;
+        const float nl = __fmaf_rn(lt.z, w, x[q]), n0 = __fmaf_rn(l2.x, w, x[q + 1]), nr = __fmaf_rn(lt.w, w, x[q + 2]);
+        const float m = fmin3(nl, n0, nr);
+        msg[kk] = fminf(m, msg_g);
+        if (AM) {
+          // the own label, then the left one, then the right one
+          int arg = (nl < n0) ? lab(kk) - 1 : lab(kk);
+          arg = (nr < fminf(nl, n0)) ? lab(kk) + 1 : arg;
+          am[kk] = (m < msg_g) ? arg : argmin_h;
+        }
+      }
+    }
+    return tail() ? 2 : 0;
+  };
+  // (the general step is kept out of the loop's way)
+  auto run = [&]() -> int {
+    for (;;) {
+      if constexpr (kRing) {
+        if (const int r = usual(Slot0{})) return r;
+      } else {
+        if ((i & 1) == 0)
+          if (const int r = usual(Slot0{})) return r;
+        if (const int r = usual(Slot1{})) return r;
+      }
+    }
+  };
+  while (run() == 1) {
+    const int j = i & 31;
+    const float* tile = taps + ((i >> 5) & 1) * tile_stride;
     const float w = tile[a.Lv * 33 + j];
-    float msg[K];
-    int am[K];
     if (delta >= L) {
       // full minimisation (lbp_min_sum_kernel.cu:88-111)
 #pragma unroll
       for (int kk = 0; kk < K; ++kk) {
-        const int t = lane + 32 * kk;
+        const int t = lab(kk);
         float m = kInf;
         int arg = 0;
         if (t < L) {
@@ -198,42 +411,20 @@ __global__ void __launch_bounds__(32 * f16_block_warps<OCC>(), OCC) lbp_forward_
         am[kk] = arg;
       }
     } else {
-      // truncated branch (lbp_min_sum_kernel.cu:112-164): the global
-      // candidate L2*w + min h, and the window terms that can beat it
-      const float L2 = tile[(a.Lv - 1) * 33 + j];
-      const float msg_g = __fmaf_rn(L2, w, pm);
+      const float msg_g = __fmaf_rn(tile[(a.Lv - 1) * 33 + j], w, pm);
       const int wcode = __float_as_int(tile[(a.Lv + 2) * 33 + j]);
       const int R = ((wcode & 0xff) != kWinGeneric) ? (wcode & 0xff) - 2 : -2;
-      float mw[K];
-      int aw[K];
-      if (R == 1) {
-        const float fm1 = tile[min(a.Lv - 1, c0 + 1) * 33 + j];  // sender t-1
-        const float f00 = tile[c0 * 33 + j];                     // sender t
-        const float fp1 = tile[max(1, c0 - 1) * 33 + j];         // sender t+1
+      const float off = tile[0 * 33 + j];
+      float fR[5];
 #pragma unroll
-        for (int kk = 0; kk < K; ++kk) {
-          const int t = lane + 32 * kk;
-          const float n0 = __fmaf_rn(f00, w, h[kk]);
-          const float nl = __fmaf_rn(fm1, w, hs[t - 1]);
-          const float nr = __fmaf_rn(fp1, w, hs[t + 1]);
-          float m = n0;
-          int arg = t;
-          m = (nl < m) ? nl : m;
-          arg = (nl < n0) ? t - 1 : arg;
-          const bool kr = nr < m;
-          mw[kk] = kr ? nr : m;
-          aw[kk] = kr ? t + 1 : arg;
-        }
-      } else if (R >= -1) {
-        // R in {-1, 0, 2}: taps of senders t-2 .. t+2 (terms beyond R skipped)
-        float fR[5];
+      for (int q = 0; q < 5; ++q) fR[q] = tile[max(1, min(a.Lv - 1, c0 - (q - 2))) * 33 + j];
 #pragma unroll
-        for (int q = 0; q < 5; ++q) fR[q] = tile[max(1, min(a.Lv - 1, c0 - (q - 2))) * 33 + j];
-#pragma unroll
-        for (int kk = 0; kk < K; ++kk) {
-          const int t = lane + 32 * kk;
-          float m = kInf;
-          int arg = 0;
+      for (int kk = 0; kk < K; ++kk) {
+        const int t = lab(kk);
+        float m = kInf;
+        int arg = 0;
+        if (R >= -1) {
+          // R in {-1, 0, 2}: taps of senders t-2 .. t+2 (terms beyond R skipped)
 #pragma unroll
           for (int q = 0; q < 5; ++q) {
             const int jd = q - 2;
@@ -242,97 +433,26 @@ __global__ void __launch_bounds__(32 * f16_block_warps<OCC>(), OCC) lbp_forward_
             m = take ? nm : m;
             arg = take ? t + jd : arg;
           }
-          mw[kk] = m;
-          aw[kk] = arg;
-        }
-      } else {
-        // generic window (offsets, wider beating ranges): the reference's
-        // rounded start / stop around t + offset
-        const float off = tile[0 * 33 + j];
-#pragma unroll
-        for (int kk = 0; kk < K; ++kk) {
-          const int t = lane + 32 * kk;
-          float m = kInf;
-          int arg = 0;
-          if (t < L) {
-            const int start = sat_u16(roundf(__fsub_rn(__fadd_rn(static_cast<float>(t - (delta - 1)), off), 1.0f)));
-            const int stop = min(sat_u16(roundf(__fadd_rn(__fadd_rn(static_cast<float>(t + delta), off), 1.0f))), L);
-            for (int s = start; s < stop; ++s) {
-              const float f = tile[max(1, min(a.Lv - 1, c0 + (t - s))) * 33 + j];
-              const float nm = __fmaf_rn(f, w, hs[s]);
-              if (nm < m) {
-                m = nm;
-                arg = s;
-              }
+        } else if (t < L) {
+          // generic window (offsets, wider beating ranges): the reference's
+          // rounded start / stop around t + offset
+          const int start = sat_u16(roundf(__fsub_rn(__fadd_rn(static_cast<float>(t - (delta - 1)), off), 1.0f)));
+          const int stop = min(sat_u16(roundf(__fadd_rn(__fadd_rn(static_cast<float>(t + delta), off), 1.0f))), L);
+          for (int s = start; s < stop; ++s) {
+            const float f = tile[max(1, min(a.Lv - 1, c0 + (t - s))) * 33 + j];
+            const float nm = __fmaf_rn(f, w, hs[s]);
+            if (nm < m) {
+              m = nm;
+              arg = s;
             }
           }
-          mw[kk] = m;
-          aw[kk] = arg;
         }
-      }
-#pragma unroll
-      for (int kk = 0; kk < K; ++kk) {
-        const bool win = mw[kk] < msg_g;
-        msg[kk] = win ? mw[kk] : msg_g;
-        am[kk] = win ? aw[kk] : argmin_h;
+        const bool win = m < msg_g;
+        msg[kk] = win ? m : msg_g;
+        am[kk] = win ? arg : argmin_h;
       }
     }
-
-    // store the row relative to the minimum of h; the chain carries the
-    // stored (half-rounded) value, so it matches memory
-    const int pq = pin + c.dpin;
-    const int64_t qo = static_cast<int64_t>(pq) * Ls;
-    __half* dstm = slot_out + qo;
-    float esum = 0.0f;
-#pragma unroll
-    for (int kk = 0; kk < K; ++kk) {
-      const __half o = __float2half_rn(msg[kk] - pm);
-      chain[kk] = __half2float(o);
-      if (lvalid(kk)) {
-        dstm[lane + 32 * kk] = o;
-        if (SCALE) esum += __expf(chain[kk]);
-      }
-    }
-    if (store_am) {
-      const int64_t ao = c.out_off + qo;
-      if (a.argmin_kind == BPL_ARGMIN_U8) {
-        uint8_t* d = static_cast<uint8_t*>(a.argmin) + ao;
-#pragma unroll
-        for (int kk = 0; kk < K; ++kk)
-          if (lvalid(kk)) d[lane + 32 * kk] = static_cast<uint8_t>(am[kk]);
-      } else if (a.argmin_kind == BPL_ARGMIN_U16) {
-        uint16_t* d = static_cast<uint16_t*>(a.argmin) + ao;
-#pragma unroll
-        for (int kk = 0; kk < K; ++kk)
-          if (lvalid(kk)) d[lane + 32 * kk] = static_cast<uint16_t>(am[kk]);
-      } else {
-        float* d = static_cast<float*>(a.argmin) + ao;
-#pragma unroll
-        for (int kk = 0; kk < K; ++kk)
-          if (lvalid(kk)) d[lane + 32 * kk] = static_cast<float>(am[kk]);
-      }
-    }
-    if (SCALE) {
-      esum = warp_sum(esum);
-      if (lane == 0) scale_out[pq] = esum;
-    }
-
-    // next tap block
-    if (j == 31 || i == nsteps - 1) {
-      __syncwarp();
-      if (32 * (b + 1) < nsteps) {
-        store_taps(a, taps + ((b + 1) & 1) * tile_stride, lane, tr, true);
-        if (32 * (b + 2) < nsteps) load_taps(a, c, b + 2, lane, nsteps, tr, true);
-      }
-    }
-    __syncwarp();  // hs is rewritten by the next step
-  };
-  for (int i0 = 0; i0 < nsteps; i0 += PF) {
-    static_for<PF>([&](auto SL) {
-      constexpr int s = decltype(SL)::value;
-      const int i = i0 + s;
-      if (i < nsteps) step(SL, i);
-    });
+    if (tail()) break;
   }
 }
 
@@ -341,16 +461,16 @@ __global__ void __launch_bounds__(32 * f16_block_warps<OCC>(), OCC) lbp_forward_
 // occupancy otherwise.
 constexpr int kF16HiOcc = 17;
 
-template <int K, bool SCALE>
+template <int NP, bool AM, int PH>
 int launch_f16_phase(const FwdArgs& a, cudaStream_t stream) {
-  auto kern = lbp_forward_f16_kernel<K, 1, SCALE, 3>;
-  int wpb = 4;
+  auto kern = lbp_forward_f16_kernel<NP, 1, AM, PH>;
+  int wpb = 4, depth = f16_depth<1>;
   if (a.nchains > kHiOccChainsPerSm * sm_count()) {
-    kern = lbp_forward_f16_kernel<K, kF16HiOcc, SCALE, 1>;
+    kern = lbp_forward_f16_kernel<NP, kF16HiOcc, AM, PH>;
     wpb = 1;
+    depth = f16_depth<kF16HiOcc>;
   }
-  const size_t per_warp = 4 * static_cast<size_t>(align4(32 * K + 2 * kHsPad) + 2 * tap_tile_rows(a.Lv) * 33);
-  const size_t smem = per_warp * wpb;
+  const size_t smem = 4 * static_cast<size_t>(f16_warp_floats(NP, depth, a.Lv)) * wpb;
   if (smem > 48 * 1024)
     BPL_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)),
                  "cudaFuncSetAttribute");
@@ -360,31 +480,23 @@ int launch_f16_phase(const FwdArgs& a, cudaStream_t stream) {
   return BPL_OK;
 }
 
-template <int K>
-int launch_f16_k(const FwdArgs& a0, cudaStream_t stream) {
+template <int NP>
+int launch_f16_pairs(const FwdArgs& a0, cudaStream_t stream) {
   FwdArgs a = a0;
-  for (int phase = 0; phase < 2; ++phase) {
-    BPL_TRACE(phase == 0 ? "lbp_forward_f16: horizontal sweeps" : "lbp_forward_f16: vertical sweeps");
-    a.phase = phase;
-    a.nchains = 2 * a.B * (phase == 0 ? a.H : a.W);
-    const int st = a.scale ? launch_f16_phase<K, true>(a, stream) : launch_f16_phase<K, false>(a, stream);
-    if (st != BPL_OK) return st;
+  const bool am = a.argmin_kind != BPL_ARGMIN_NONE;
+  a.nchains = 2 * a.B * a.H;
+  int st;
+  {
+    BPL_TRACE("lbp_forward_f16: horizontal sweeps");
+    st = am ? launch_f16_phase<NP, true, 0>(a, stream) : launch_f16_phase<NP, false, 0>(a, stream);
   }
-  return BPL_OK;
+  if (st != BPL_OK) return st;
+  a.nchains = 2 * a.B * a.W;
+  BPL_TRACE("lbp_forward_f16: vertical sweeps");
+  return am ? launch_f16_phase<NP, true, 1>(a, stream) : launch_f16_phase<NP, false, 1>(a, stream);
 }
 
-inline int dispatch_f16(const FwdArgs& a, cudaStream_t s) {
-  switch ((a.L + 31) / 32) {
-    case 1: return launch_f16_k<1>(a, s);
-    case 2: return launch_f16_k<2>(a, s);
-    case 3: return launch_f16_k<3>(a, s);
-    case 4: return launch_f16_k<4>(a, s);
-    case 5: return launch_f16_k<5>(a, s);
-    case 6: return launch_f16_k<6>(a, s);
-    case 7: return launch_f16_k<7>(a, s);
-    case 8: return launch_f16_k<8>(a, s);
-    default: return set_error(BPL_ERR_UNSUPPORTED, "lbp_forward_f16: the lean kernel serves L <= 256");
-  }
-}
+int lbp_forward_f16_pairs3(const FwdArgs& a, cudaStream_t s);
+int lbp_forward_f16_pairs4(const FwdArgs& a, cudaStream_t s);
 
 }  // namespace bpl
