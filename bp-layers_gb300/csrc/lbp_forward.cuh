@@ -443,21 +443,21 @@ constexpr int kHiOcc = 17;
 template <int OCC>
 constexpr int fwd_block_warps() { return (OCC > 1) ? 1 : 4; }
 
+// min over v[0 .. N-1], three at a time
+template <int N>
+__device__ __forceinline__ float min_of(const float* v) {
+  if constexpr (N == 1) {
+    return v[0];
+  } else if constexpr (N == 2) {
+    return fminf(v[0], v[1]);
+  } else {
+    constexpr int A = (N + 2) / 3, B = (N - A + 1) / 2;
+    return fmin3(min_of<A>(v), min_of<B>(v + A), min_of<N - A - B>(v + A + B));
+  }
+}
 // min over a lane's label slots
 template <int K>
-__device__ __forceinline__ float slot_min(const float (&v)[K]) {
-  float m[K];
-#pragma unroll
-  for (int k = 0; k < K; ++k) m[k] = v[k];
-#pragma unroll
-  for (int n = K; n > 1; n = (n + 2) / 3) {
-#pragma unroll
-    for (int k = 0; k < (n + 2) / 3; ++k)
-      m[k] = (3 * k + 2 < n) ? fmin3(m[3 * k], m[3 * k + 1], m[(3 * k + 2 < n) ? 3 * k + 2 : 0])
-             : (3 * k + 1 < n) ? fminf(m[3 * k], m[(3 * k + 1 < n) ? 3 * k + 1 : 0]) : m[3 * k];
-  }
-  return m[0];
-}
+__device__ __forceinline__ float slot_min(const float (&v)[K]) { return min_of<K>(v); }
 
 // The instantiations whose step has the lean form (see store_lean).
 template <int K, int VARIANT, int NW, typename T>
