@@ -163,8 +163,17 @@ __global__ void __launch_bounds__(256) beliefs_bwd_kernel(const T* msgs, const T
     }
   }
   if (gT != nullptr) {
-    tacc = warp_sum(tacc);
-    if (lane == 0 && tacc != 0.0f) atomicAdd(gT, tacc);
+    // warps' sums joined in double, one atomic per block: an eighth of the
+    // float additions in run-dependent order
+    __shared__ double s_t[8];
+    const float wt = warp_sum(tacc);
+    if (lane == 0) s_t[threadIdx.x >> 5] = wt;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      double t = s_t[0];
+      for (int q = 1; q < 8; ++q) t += s_t[q];
+      if (t != 0.0) atomicAdd(gT, static_cast<float>(t));
+    }
   }
 }
 
