@@ -226,9 +226,12 @@ class LBPMinSumLoop(torch.autograd.Function):
     def _recompute_backward(ctx, in_grad):
         cost, cost_h, taps, edge, messages, vert0 = ctx.saved_tensors
         half, L, delta = ctx.half, ctx.L, ctx.delta
-        # the state before the first pass: the final messages with the
-        # initial vertical slots back (see the class docstring)
-        m = messages.detach().clone()
+        # the state before the first pass (see the class docstring): the
+        # initial vertical slots and the horizontal slots at the borders no
+        # pass writes; the rest of those is written before it is read
+        m = torch.empty_like(messages)
+        m[:, LEFT, :, 0] = messages[:, LEFT, :, 0]
+        m[:, RIGHT, :, -1] = messages[:, RIGHT, :, -1]
         m[:, UP:DOWN + 1] = vert0
         B, _, H, W, Ls = m.shape
         am = torch.empty((B, 4, H, W, Ls), dtype=ctx.am_dtype, device=m.device)
@@ -252,17 +255,19 @@ class LBPMinSumLoop(torch.autograd.Function):
                 gc, gtaps, ge = acc(gc, c_k), acc(gtaps, t_k), acc(ge, e_k)
             return gc, gtaps, ge, g
         g_in = in_grad
+        # the passes add their cost gradients onto one volume, binned for the
+        # packed taps' fold (as BPLayerFn's single launch does)
+        gc = torch.zeros((B, H, W, Ls), device=m.device)
         for _ in range(ctx.iters):
             if half:
                 ops.lbp_forward_f16(ops.LBP_STEREO, cost_h, taps, edge, m, delta, L, argmin=am)
-                c_k, t_k, e_k = ops.lbp_backward_passes(ops.LBP_STEREO, taps, edge, g_in, messages, am.unsqueeze(0),
-                                                        None, L=L, workspace=ws)
             else:
                 ops.lbp_forward(ops.LBP_STEREO, cost, taps, edge, m, delta, argmin_dtype=ctx.am_dtype, argmin=am,
                                 scale=sc)
-                c_k, t_k, e_k = ops.lbp_backward_passes(ops.LBP_STEREO, taps, edge, g_in, messages, am.unsqueeze(0),
-                                                        sc.unsqueeze(0), L=L, workspace=ws)
-            gc, gtaps, ge = acc(gc, c_k), acc(gtaps, t_k), acc(ge, e_k)
+            _, t_k, e_k = ops.lbp_backward_passes(ops.LBP_STEREO, taps, edge, g_in, messages, am.unsqueeze(0),
+                                                  None if half else sc.unsqueeze(0), L=L, workspace=ws,
+                                                  grad_cost_into=gc, cost_sign=1.0, layer_taps=taps.shape[2] == 6)
+            gtaps, ge = acc(gtaps, t_k), acc(ge, e_k)
         return gc, gtaps, ge, in_grad
 
 
