@@ -290,10 +290,12 @@ class BPLayerFn(torch.autograd.Function):
     beliefs' backward also writes the adjoint's in_grad (for a leaf message
     tensor the materialised message gradient) in the same pass, and takes
     z/T for the temperature's gradient from the beliefs and one float per
-    pixel the forward keeps, instead of re-reading messages and cost."""
+    pixel the forward keeps, instead of re-reading messages and cost.
+    keep=False (gradients are off when the layer is called): nothing is kept
+    for a backward, so the passes store no indices."""
 
     @staticmethod
-    def forward(ctx, prob_vol, edge, messages, affinities, offset, T, iters, delta):
+    def forward(ctx, prob_vol, edge, messages, affinities, offset, T, iters, delta, keep=True):
         ctx.set_materialize_grads(False)
         taps = pack_affinities(affinities, offset)
         half = messages.dtype == torch.float16
@@ -302,6 +304,16 @@ class BPLayerFn(torch.autograd.Function):
         Ls = messages.shape[-1]
         am_dtype = torch.uint8 if L <= 256 else torch.int16
         cost = ops.half_padded(prob, -1.0) if half else -prob
+        if not keep:
+            # gradients are off: no indices, no per-pass scales
+            scale = None if half else torch.empty((B, 4, H, W), dtype=torch.float32, device=prob.device)
+            for _ in range(iters):
+                if half:
+                    ops.lbp_forward_f16(ops.LBP_STEREO, cost, taps, edge, messages, int(delta), L, argmin_dtype=None)
+                else:
+                    ops.lbp_forward(ops.LBP_STEREO, cost, taps, edge, messages, int(delta), argmin_dtype=None,
+                                    scale=scale)
+            return ops.beliefs_forward_any_cost(messages, prob, T, L, cost_sign=-1.0), messages
         argmins = torch.empty((iters, B, 4, H, W, Ls), dtype=am_dtype, device=prob.device)
         # FP16: no scales (the adjoint normalises from the final rows)
         scales = None if half else torch.empty((iters, B, 4, H, W), dtype=torch.float32, device=prob.device)
@@ -352,7 +364,7 @@ class BPLayerFn(torch.autograd.Function):
         gm = None
         if need_m:
             gm = ops.leaf_message_grad(gin) if ctx.leaf_messages else gin
-        return gprob, ge, gm, g_aff, g_off, (gT.view_as(T) if gT is not None else None), None, None
+        return gprob, ge, gm, g_aff, g_off, (gT.view_as(T) if gT is not None else None), None, None, None
 
 
 class MessagePassing(nn.Module):
@@ -428,7 +440,7 @@ class MessagePassing(nn.Module):
         fused = self.fused and self.adjoint == "reference" and not self.recompute_argmin and self.max_iter >= 1
         if fused and self.storage == "fp32":
             return BPLayerFn.apply(prob_vol, edge_weights, messages, affinities, offset, self.softmin.T,
-                                   self.max_iter, self.delta)
+                                   self.max_iter, self.delta, torch.is_grad_enabled())
         if self.storage == "fp16":
             if messages is None or messages.dtype != torch.float16:
                 # a half copy of the caller's start (or zeros): no gradient
@@ -439,7 +451,7 @@ class MessagePassing(nn.Module):
                 messages = m
             if fused:
                 return BPLayerFn.apply(prob_vol, edge_weights, messages, affinities, offset, self.softmin.T,
-                                       self.max_iter, self.delta)
+                                       self.max_iter, self.delta, torch.is_grad_enabled())
             cost = -prob_vol
             cost_h = ops.to_half_padded(cost.detach(), C)
             messages = LBPMinSumLoop.apply(cost, cost_h, edge_weights, messages, self.delta, affinities, offset,
