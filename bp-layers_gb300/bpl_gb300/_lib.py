@@ -49,6 +49,7 @@ SIGNATURES = {
     "bpl_messages_argmin": [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int] + [c_int] * 6 + [c_void_p],
     "bpl_beliefs_infer": [c_void_p, c_int, c_int, c_void_p] + [c_int] * 4 + [c_void_p],
     "bpl_pack_taps": [c_void_p] * 3 + [c_int] * 4 + [c_void_p],
+    "bpl_scalar_taps": [c_void_p] * 3 + [c_int] * 3 + [c_void_p],
     "bpl_unpack_tap_grad": [c_void_p] * 3 + [c_int] * 4 + [c_void_p],
     "bpl_lbp_backward_noalloc": [c_int] + [c_void_p] * 5 + [c_int] + [c_void_p] * 4 + [c_int] * 7 + [c_void_p],
 }

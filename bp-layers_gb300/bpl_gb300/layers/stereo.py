@@ -292,12 +292,18 @@ class BPLayerFn(torch.autograd.Function):
     z/T for the temperature's gradient from the beliefs and one float per
     pixel the forward keeps, instead of re-reading messages and cost.
     keep=False (gradients are off when the layer is called): nothing is kept
-    for a backward, so the passes store no indices."""
+    for a backward, so the passes store no indices; the taps of the default
+    affinities may then come straight from the scalars L1, L2 (affinities and
+    offset None)."""
 
     @staticmethod
-    def forward(ctx, prob_vol, edge, messages, affinities, offset, T, iters, delta, keep=True):
+    def forward(ctx, prob_vol, edge, messages, affinities, offset, T, iters, delta, keep=True, L1=None, L2=None):
         ctx.set_materialize_grads(False)
-        taps = pack_affinities(affinities, offset)
+        if affinities is None:
+            N, H, W, _ = prob_vol.shape
+            taps = ops.scalar_taps(L1, L2, N, H, W)
+        else:
+            taps = pack_affinities(affinities, offset)
         half = messages.dtype == torch.float16
         prob = prob_vol.contiguous()
         B, H, W, L = prob.shape
@@ -364,7 +370,8 @@ class BPLayerFn(torch.autograd.Function):
         gm = None
         if need_m:
             gm = ops.leaf_message_grad(gin) if ctx.leaf_messages else gin
-        return gprob, ge, gm, g_aff, g_off, (gT.view_as(T) if gT is not None else None), None, None, None
+        return gprob, ge, gm, g_aff, g_off, (gT.view_as(T) if gT is not None else None), None, None, None, \
+            None, None
 
 
 class MessagePassing(nn.Module):
@@ -425,9 +432,16 @@ class MessagePassing(nn.Module):
     def forward(self, prob_vol, edge_weights, affinities, offset, messages):
         N, H, W, C = prob_vol.shape
         dev = prob_vol.device
+        fused = self.fused and self.adjoint == "reference" and not self.recompute_argmin and self.max_iter >= 1
         if edge_weights is None:
             edge_weights = torch.ones((N, 4, H, W), device=dev)
-        if affinities is None:
+        # gradients off and the default affinities: the taps from the scalars
+        scalars = ()
+        if fused and affinities is None and offset is None and not torch.is_grad_enabled() and all(
+                isinstance(v, torch.Tensor) and v.device == dev and v.is_cuda and v.dtype == torch.float32
+                and v.numel() == 1 for v in (self._L1, self._L2)):
+            scalars = (self._L1, self._L2)
+        elif affinities is None:
             if (self._L1 is not None) and (self._L2 is not None):
                 affinities = torch.zeros((N, 4, 3, H, W), dtype=torch.float, device=dev)
                 affinities[:, :, :2, :, :] = self._L1
@@ -435,12 +449,11 @@ class MessagePassing(nn.Module):
         else:
             if (self._L1 is not None and self._L2 is None) or (self._L1 is None and self._L2 is not None):
                 raise ValueError("L1 or L2 is None and affinities are not set!")
-        if offset is None:
+        if offset is None and not scalars:
             offset = torch.zeros((N, 4, H, W), device=dev)
-        fused = self.fused and self.adjoint == "reference" and not self.recompute_argmin and self.max_iter >= 1
         if fused and self.storage == "fp32":
             return BPLayerFn.apply(prob_vol, edge_weights, messages, affinities, offset, self.softmin.T,
-                                   self.max_iter, self.delta, torch.is_grad_enabled())
+                                   self.max_iter, self.delta, torch.is_grad_enabled(), *scalars)
         if self.storage == "fp16":
             if messages is None or messages.dtype != torch.float16:
                 # a half copy of the caller's start (or zeros): no gradient
@@ -451,7 +464,7 @@ class MessagePassing(nn.Module):
                 messages = m
             if fused:
                 return BPLayerFn.apply(prob_vol, edge_weights, messages, affinities, offset, self.softmin.T,
-                                       self.max_iter, self.delta, torch.is_grad_enabled())
+                                       self.max_iter, self.delta, torch.is_grad_enabled(), *scalars)
             cost = -prob_vol
             cost_h = ops.to_half_padded(cost.detach(), C)
             messages = LBPMinSumLoop.apply(cost, cost_h, edge_weights, messages, self.delta, affinities, offset,

@@ -745,6 +745,19 @@ def pack_taps(affinities: torch.Tensor, offset: torch.Tensor) -> torch.Tensor:
     return taps
 
 
+def scalar_taps(L1: torch.Tensor, L2: torch.Tensor, N: int, H: int, W: int) -> torch.Tensor:
+    """(N,4,6,H,W) taps of scalar affinities [L1, L1, L2] (one-element float
+    CUDA tensors) and no offset, one launch."""
+    for nm, t in (("L1", L1), ("L2", L2)):
+        _check_input(nm, t)
+        if t.numel() != 1:
+            raise BplError(f"{nm} must have one element")
+    taps = torch.empty((N, 4, 6, H, W), dtype=torch.float32, device=L1.device)
+    st = _timed("scalar_taps", lambda: lib().bpl_scalar_taps(_ptr(L1), _ptr(L2), _ptr(taps), N, H, W, _stream(L1)))
+    check(st, "bpl_scalar_taps")
+    return taps
+
+
 def unpack_tap_grad(grad_taps: torch.Tensor):
     """Gradient fold of pack_taps: (grad_affinities (N,4,K,H,W), grad_offset
     (N,4,H,W)), one kernel pass (message_passing_op_cuda.py:75-93)."""

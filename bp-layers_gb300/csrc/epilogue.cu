@@ -166,6 +166,26 @@ __global__ void pack_taps_kernel(const float* __restrict__ aff, const float* __r
   }
 }
 
+// The taps of scalar affinities [L1, L1, L2] and no offset, the layer's
+// default (message_passing_op_cuda.py:145-158): [0, L2, L1, 0, L1, L2] at
+// every pixel and direction, from the two scalars in one launch instead of
+// two zero fills, two broadcasts and the packing (24x32x32 inference, launch
+// bound: 0.25 -> 0.15 ms with the rest of the gradient-free path).
+__global__ void scalar_taps_kernel(const float* __restrict__ L1, const float* __restrict__ L2,
+                                   float* __restrict__ taps, int64_t HW, int64_t total) {
+  const float l1 = __ldg(L1), l2 = __ldg(L2);
+  for (int64_t e = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; e < total;
+       e += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    float* t = taps + (e / HW) * 6 * HW + e % HW;
+    t[0] = 0.0f;
+    t[HW] = l2;
+    t[2 * HW] = l1;
+    t[3 * HW] = 0.0f;
+    t[4 * HW] = l1;
+    t[5 * HW] = l2;
+  }
+}
+
 // the fold of the tap gradient (message_passing_op_cuda.py:75-93): each
 // affinity sums the gradients of the taps it fills (L3: taps 1 and Kp-1,
 // added in that order), the offset takes tap 0, the centre tap is dropped
@@ -301,6 +321,17 @@ extern "C" int bpl_pack_taps(const float* affinities, const float* offset, float
   const unsigned blocks = static_cast<unsigned>(std::min<int64_t>((total + 255) / 256, 152 * 16));
   pack_taps_kernel<<<blocks, 256, 0, as_stream(stream)>>>(affinities, offset, taps, N, K, HW);
   BPL_CUDA_TRY(cudaGetLastError(), "pack_taps launch");
+  return BPL_OK;
+}
+
+extern "C" int bpl_scalar_taps(const float* L1, const float* L2, float* taps, int N, int H, int W, void* stream) {
+  BPL_TRACE("bpl_scalar_taps");
+  BPL_REQUIRE(L1 && L2 && taps, "scalar_taps: null pointer");
+  BPL_REQUIRE(N >= 1 && H >= 1 && W >= 1, "scalar_taps: bad shape");
+  const int64_t HW = static_cast<int64_t>(H) * W, total = static_cast<int64_t>(N) * 4 * HW;
+  const unsigned blocks = static_cast<unsigned>(std::min<int64_t>((total + 255) / 256, 152 * 16));
+  scalar_taps_kernel<<<blocks, 256, 0, as_stream(stream)>>>(L1, L2, taps, HW, total);
+  BPL_CUDA_TRY(cudaGetLastError(), "scalar_taps launch");
   return BPL_OK;
 }
 

@@ -364,7 +364,14 @@ int bpl_pack_taps(const float* affinities, const float* offset, float* taps, int
                   void* stream);
 
 /*
- * Its gradient fold (message_passing_op_cuda.py:75-93): grad_affinities
+ * The taps of the layer's default affinities [L1, L1, L2] (L1, L2: one float
+ * each, on the device) and no offset (message_passing_op_cuda.py:145-158):
+ * taps (N,4,6,H,W) [0, L2, L1, 0, L1, L2].
+ */
+int bpl_scalar_taps(const float* L1, const float* L2, float* taps, int N, int H, int W, void* stream);
+
+/*
+ * bpl_pack_taps' gradient fold (message_passing_op_cuda.py:75-93): grad_affinities
  * (N,4,K,H,W), each affinity the gradient of the taps it fills (L3: taps 1
  * and K+2), and grad_offset (N,4,H,W) = tap 0's.
  */

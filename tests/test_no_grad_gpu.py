@@ -39,3 +39,15 @@ def test_values_and_gradients(storage, L):
     assert torch.equal(b0, b1) and torch.equal(m0, m1) and not b1.requires_grad
     assert torch.equal(b0, b2) and torch.equal(m0, m2)
     assert float((g2 - g0).abs().max()) <= 1e-5 * float(g0.abs().max())
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 1), (2, 3, 5), (1, 33, 70)])
+def test_scalar_taps_equal_the_packing(shape):
+    from bpl_gb300 import ops
+    dev = torch.device("cuda:0")
+    N, H, W = shape
+    L1, L2 = torch.tensor(0.125, device=dev), torch.tensor(2.5, device=dev)
+    aff = torch.zeros((N, 4, 3, H, W), device=dev)
+    aff[:, :, :2] = L1
+    aff[:, :, 2] = L2
+    assert torch.equal(ops.scalar_taps(L1, L2, N, H, W), ops.pack_taps(aff, torch.zeros((N, 4, H, W), device=dev)))
