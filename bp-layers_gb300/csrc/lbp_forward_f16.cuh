@@ -17,14 +17,13 @@
 //     is at least the candidate's, the "tie-only" offsets of the FP32 kernel)
 //     are not evaluated at all;
 //   * the per-message scale (the sum of exp of the stored row) is computed
-//     only when the caller asks for it (SCALE), off the chain.
+//     only when the caller asks for it, off the chain.
 // All arithmetic is FP32 (cost and messages are converted when loaded); the
 // rounding of each stored message to half is the only FP16 operation.
 //
 // Reference semantics followed (sweep order, h, window, candidate):
 // ops/lbp_stereo/src/lbp_min_sum_kernel.cu:55-164.
 #pragma once
-
 
 #include <type_traits>
 
