@@ -142,8 +142,9 @@ __global__ void __launch_bounds__(MAXT, MINB) flow_forward_kernel(FlowArgs a) {
     if (BULK) {
       // every warp issues its share of the rows: one thread issuing all of
       // them made its warp the last at each row's barrier (384x512, 32
-      // channels, window 65: 3.43 -> 3.28 ms).  Thread 0's arrival is the phase's only one, so the phase cannot
-      // end before it, whichever warp's copies land first
+      // channels, window 65, with the backward: 4.97 -> 4.82 ms).  Thread 0's arrival is the
+      // phase's only one, so the phase cannot end before it, whichever warp's
+      // copies land first
       if (lane == 0) {
         fence_proxy_async();
         const uint32_t rb = (b_hi > b_lo) ? static_cast<uint32_t>(b_hi - b_lo) * 4u : 0u;
@@ -240,7 +241,7 @@ __global__ void __launch_bounds__(MAXT, MINB) flow_forward_kernel(FlowArgs a) {
     // two 3-input minima and the first one equal to the result: the start
     // (9999999, 0) is in the final minimum, so what the index is when no value
     // is below it does not matter.  With the warps taking turns at the
-    // row's result below, 3.28 -> 3.15 ms at 384x512, 32 channels, window 65.
+    // row's result below, 4.82 -> 4.69 ms for the same call (3.25 ms of it here).
     unsigned long long key[4];
     auto running = [&](float val, int i, int j) {
       if (val < mn[i][j]) {
