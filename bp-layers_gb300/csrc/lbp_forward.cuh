@@ -1533,9 +1533,13 @@ int launch_phase(const FwdArgs& a0, cudaStream_t stream) {
   // chains per block: up to wmax warps while the block fits in 200 KB
   const int cpb = std::max(1, std::min(wmax / NW, static_cast<int>((200 * 1024) / per_chain)));
   const size_t smem = per_chain * cpb;
-  if (smem > 48 * 1024) {
-    if (static_cast<int>(smem) > max_smem_optin())
-      return set_error(BPL_ERR_UNSUPPORTED, "lbp_forward: shared memory %zu exceeds device limit", smem);
+  // the kernel's static tables count against both limits: the 48 KB a launch
+  // may use by default and the opt-in maximum
+  constexpr size_t kStatic =
+      sizeof(T) == 4 ? sizeof(crm::Tables) : sizeof(crm::ExpEntry) + sizeof(crm::LogEntry) + sizeof(float4);
+  if (smem + kStatic > 48 * 1024) {
+    if (static_cast<int>(smem + kStatic) > max_smem_optin())
+      return set_error(BPL_ERR_UNSUPPORTED, "lbp_forward: shared memory %zu exceeds device limit", smem + kStatic);
     BPL_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)),
                  "cudaFuncSetAttribute");
   }
