@@ -947,7 +947,7 @@ __global__ void __launch_bounds__(32 * fwd_block_warps<OCC>(), OCC) lbp_forward_
       int lcnt = 0, llab = 0;
 #pragma unroll
       for (int kk = 0; kk < KW; ++kk) {
-        const bool eq = h[kk] == pm;
+        const bool eq = lvalid(kk) && h[kk] == pm;  // (a row of NaNs: the minimum is that of no label)
         lcnt += eq ? 1 : 0;
         llab = eq ? c.t0 + lane + 32 * kk : llab;
       }
@@ -1145,8 +1145,9 @@ __global__ void __launch_bounds__(32 * fwd_block_warps<OCC>(), OCC) lbp_forward_
           }
       }
       // exact ties of the minimum: the reference tree picks the label (and,
-      // between -0 and +0, the value)
-      if (tot > 1) {
+      // between -0 and +0, the value); so it does where no label has it, a
+      // row of NaNs
+      if (tot != 1) {
         float tv[K];
         int tl[K];
 #pragma unroll
@@ -1159,6 +1160,9 @@ __global__ void __launch_bounds__(32 * fwd_block_warps<OCC>(), OCC) lbp_forward_
         min_h = cs.hs[argmin_h];
       }
       const float msg_g = __fmaf_rn(L2, w, min_h);
+      // The forms below read h outside [0, L) as +inf, which reaches no
+      // finite candidate; the scan of a candidate that is none is clipped.
+      const bool finite_g = msg_g < kInf;
 
       // Fast form (one warp per scanline, stereo zero-offset windows whose
       // beating offsets are |jd| <= R): the 2R+1 terms for every label, and
@@ -1174,7 +1178,7 @@ __global__ void __launch_bounds__(32 * fwd_block_warps<OCC>(), OCC) lbp_forward_
       // only sends the step to the full scan (several senders) or names the
       // one sender s1 for the fix.
       int nn = 0, smax = -1;
-      if (NW == 1 && stereo) {
+      if (NW == 1 && stereo && finite_g) {
         wcode = __float_as_int(tile[(a.Lv + 2) * 33 + j]);
         if ((wcode & 0xff) != kWinGeneric) {
           R = (wcode & 0xff) - 2;
@@ -1283,7 +1287,7 @@ __global__ void __launch_bounds__(32 * fwd_block_warps<OCC>(), OCC) lbp_forward_
           }
         }
       } else {
-        const bool fast = stereo && delta <= kFastDelta && off == 0.0f;
+        const bool fast = stereo && delta <= kFastDelta && off == 0.0f && finite_g;
         // taps of the zero-offset window: the tap of sender s = t + jd is
         // clamp(Lv/2 - jd, 1, Lv-1), the same for every label
         float fj[2 * kFastDelta + 1];
@@ -1301,8 +1305,7 @@ __global__ void __launch_bounds__(32 * fwd_block_warps<OCC>(), OCC) lbp_forward_
           float m = kInf;
           int arg = 0;
           if (fast && delta == 3) {
-            // hs holds +inf outside [0, L), which never wins against the
-            // finite global candidate, in place of the clipping
+            // hs holds +inf outside [0, L), in place of the clipping (finite_g)
 #pragma unroll
             for (int q = kFastDelta - 3; q <= kFastDelta + 3; ++q) {
               const float nm = __fmaf_rn(fj[q], w, cs.hs[t + q - kFastDelta]);

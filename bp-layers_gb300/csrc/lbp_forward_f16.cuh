@@ -273,9 +273,11 @@ __global__ void __launch_bounds__(32 * f16_block_warps<OCC>(), OCC) lbp_forward_
     __syncwarp();  // h of the whole pixel is visible in hs
     issue(SL, i + (kRing ? DEPTH - 1 : 2));  // (ring: over the rows of step i - 1, which every lane is past)
     if (AM) {
-      int ll = -1;
+      // (label 0 where no label's h equals the minimum, a row of NaNs: the
+      // adjoint adds at this index, so it has to be a label)
+      int ll = 0;
 #pragma unroll
-      for (int kk = 0; kk < K; ++kk) ll = (h[kk] == pm) ? lab(kk) : ll;
+      for (int kk = 0; kk < K; ++kk) ll = (lvalid(kk) && h[kk] == pm) ? lab(kk) : ll;
       argmin_h = __reduce_max_sync(FULL, ll);
     }
   };
