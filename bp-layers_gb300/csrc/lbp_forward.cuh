@@ -727,9 +727,10 @@ __global__ void __launch_bounds__(32 * fwd_block_warps<OCC>(), OCC) lbp_forward_
       // second sender within rounding of the candidate, a window term equal
       // to the candidate or to 0 (ties and their signs), several labels
       // below the candidate in a lane or one in every lane, a rounding of
-      // exp or log that is undecided, a NaN or infinity, or a record of
-      // another form; that step runs the code after the loop, which is kept
-      // out of the hot loop's way.  WIDE: taps at distance 2 below L2.
+      // exp or log that is undecided, an infinite minimum or candidate, or a
+      // record of another form; that step runs the code after the loop, which
+      // is kept out of the hot loop's way.  (A NaN term is dropped here as by
+      // the forms there: no minimum and no vote sees it.)  WIDE: taps at distance 2 below L2.
       // (Moving the stores and the next step's h before the vote, to overlap
       // it, gained 2 % on the latency-bound launch and lost 3 % on the
       // others.)
@@ -1152,7 +1153,7 @@ __global__ void __launch_bounds__(32 * fwd_block_warps<OCC>(), OCC) lbp_forward_
         int tl[K];
 #pragma unroll
         for (int k = 0; k < K; ++k) {
-          tv[k] = cs.hs[lane + 32 * k];
+          tv[k] = fminf(cs.hs[lane + 32 * k], kInf);  // (a NaN beats nothing)
           tl[k] = lane + 32 * k;
         }
         float mv;
@@ -1211,16 +1212,17 @@ __global__ void __launch_bounds__(32 * fwd_block_warps<OCC>(), OCC) lbp_forward_
 #pragma unroll
           for (int kk = 0; kk < KW; ++kk) {
             const int t = c.t0 + lane + 32 * kk;
-            // increasing sender order, `<=`: the last minimiser wins
-            float m = __fmaf_rn(fm1, w, cs.hs[t - 1]);
+            // increasing sender order, `<=`: the last minimiser wins, a NaN
+            // term never (fminf drops it)
+            const float m = fminf(__fmaf_rn(fm1, w, cs.hs[t - 1]), kInf);
             int arg = t - 1;
             const float n0 = __fmaf_rn(f00, w, h[kk]);
             const float n1 = __fmaf_rn(fp1, w, cs.hs[t + 1]);
             const bool k0 = n0 <= m;
-            m = k0 ? n0 : m;
+            const float m0 = k0 ? n0 : m;
             arg = k0 ? t : arg;
-            const bool k1 = n1 <= m;
-            mw[kk] = k1 ? n1 : m;
+            const bool k1 = n1 <= m0;
+            mw[kk] = k1 ? n1 : m0;
             aw[kk] = k1 ? t + 1 : arg;
           }
         } else if (R >= 0) {

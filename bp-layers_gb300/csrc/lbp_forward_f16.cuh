@@ -366,9 +366,9 @@ __global__ void __launch_bounds__(32 * f16_block_warps<OCC>(), OCC) lbp_forward_
         const float m = fmin3(nl, n0, nr);
         msg[kk] = fminf(m, msg_g);
         if (AM) {
-          // the own label, then the left one, then the right one
-          int arg = (nl < n0) ? lab(kk) - 1 : lab(kk);
-          arg = (nr < fminf(nl, n0)) ? lab(kk) + 1 : arg;
+          // the own label, then the left one, then the right one (by equality
+          // with the minimum: a NaN term is none of them)
+          const int arg = (n0 == m) ? lab(kk) : (nl == m) ? lab(kk) - 1 : lab(kk) + 1;
           am[kk] = (m < msg_g) ? arg : argmin_h;
         }
       }

@@ -60,3 +60,51 @@ def test_f32_indices_are_labels(kind, delta, L):
     _, am, _ = ops.lbp_forward(0, c, t, e, m, delta, argmin_dtype=torch.float32)
     am = am.cpu().numpy()
     assert am.min() >= 0 and am.max() < L
+
+
+def _holes(g, cost):
+    """One or two labels per pixel lost, beside the pixel's smallest cost and
+    anywhere; the copy with +inf in their place."""
+    B, H, W, L = cost.shape
+    gap = np.zeros(cost.shape, bool)
+    low = cost.argmin(-1)
+    b, y, x = np.indices(low.shape)
+    gap[b, y, x, np.clip(low + g.choice([-1, 1, 2], size=low.shape), 0, L - 1)] = True
+    gap[b, y, x, g.integers(0, L, size=low.shape)] = True
+    gap[b, y, x, low] = False
+    gap &= g.random(low.shape)[..., None] < 0.5
+    return np.where(gap, np.nan, cost).astype(np.float32), np.where(gap, np.inf, cost).astype(np.float32)
+
+
+@pytest.mark.parametrize("L", [5, 33, 64, 130])
+def test_f16_nan_terms_are_skipped(L):
+    from test_f16_pairs_gpu import _emulate
+    g, cost, edge, taps = _f16_inputs(2, 6, 9, L, 7 + L)
+    nan, inf = _holes(g, cost)
+    m, am = _f16_run(nan, edge, taps, L, torch.uint8)
+    ref = np.zeros(m.shape, np.float32)
+    with np.errstate(invalid="ignore"):
+        ra = _emulate(inf, taps, edge, ref, L)
+    np.testing.assert_array_equal(m, ref)
+    np.testing.assert_array_equal(am, ra)
+
+
+@pytest.mark.parametrize("form", ["lean", "own tap", "8 taps", "offset"])
+@pytest.mark.parametrize("L", [5, 33, 96, 192])
+def test_f32_nan_terms_are_skipped(form, L):
+    """Steps of the hot loop and of the forms outside it alike."""
+    import cases
+    import oracle
+    from test_lbp_forward_gpu import _run_gpu, assert_parity
+    g, cost, edge, taps = _f16_inputs(2, 6, 40, L, 11 + L)
+    if form == "own tap":
+        taps[:, :, 3] = 0.03125
+    elif form == "8 taps":
+        taps = cases.random_taps8(g, 2, 6, 40)
+    elif form == "offset":
+        taps[:, :, 0] = 0.75
+    nan, inf = _holes(g, (4.0 * cost).astype(np.float32))
+    msgs = np.zeros((2, 4, 6, 40, L), np.float32)
+    with np.errstate(invalid="ignore"):
+        ref = oracle.lbp_forward(0, inf, taps, edge, msgs, 3)
+    assert_parity(_run_gpu(0, nan, taps, edge, msgs, 3, 1), ref, form)
