@@ -42,11 +42,14 @@ struct SadArgs {
   const float* f1;
   float* out;
   int B, C, H, W, D;
+  int g0, n;      // disparities of this launch: n from index g0 (a multiple of kPD) of the volume's D
   int min_disp;
   float step;
   int unit_step;  // step == 1: d = di + min_disp
-  int dlo, dhi;   // smallest / largest disparity
+  int dlo, dhi;   // smallest / largest disparity of the launch
 };
+
+constexpr int kMaxD = 256;  // disparities per launch (the largest block has 512 threads)
 
 __device__ __forceinline__ int disparity(const SadArgs& a, int di) {
   if (a.unit_step) return di + a.min_disp;
@@ -65,7 +68,7 @@ constexpr int kPXG = kTX / kPX;  // pixel groups per block
 // leading pad of an f1 row: (window start + pad) % 4 == 0 for every thread
 __host__ __device__ inline int sad_pad(int dhi, int dlo) { return ((7 - (dhi - dlo)) % 4 + 4) % 4; }
 
-// grid (ceil(W/kTX), H, B); block kPXG x (D/kPD rounded up) threads.
+// grid (ceil(W/kTX), H, B); block kPXG x (n/kPD rounded up) threads.
 // MAXT/MINB: blocks of up to 384 threads run with registers capped (80, no
 // spills) so that 2-3 blocks stay resident per SM and one block's chunk
 // barrier does not idle the SM; 512-thread blocks (D > 192) keep theirs.
@@ -78,7 +81,7 @@ __global__ void __launch_bounds__(MAXT, MINB) sad_forward_kernel(SadArgs a) {
   const int spanp = (pad + span + 3) & ~3;
   const int bufsz = kCChunk * (kTX + spanp);   // one chunk: s0 [kCChunk][kTX], s1 [kCChunk][spanp]
   const int xb = x0 - a.dhi - pad;             // f1 column of s1[.][0]
-  const int ndg = (a.D + kPD - 1) / kPD;
+  const int ndg = (a.n + kPD - 1) / kPD;
   const int tid = threadIdx.x;
   const int nthreads = blockDim.x;
   const int xg = tid % kPXG;                   // pixel group
@@ -90,7 +93,7 @@ __global__ void __launch_bounds__(MAXT, MINB) sad_forward_kernel(SadArgs a) {
 
   int dv[kPD];
 #pragma unroll
-  for (int q = 0; q < kPD; ++q) dv[q] = disparity(a, min(dg * kPD + q, a.D - 1));
+  for (int q = 0; q < kPD; ++q) dv[q] = disparity(a, a.g0 + min(dg * kPD + q, a.n - 1));
   float acc[kPX][kPD];
 #pragma unroll
   for (int p = 0; p < kPX; ++p)
@@ -194,14 +197,14 @@ __global__ void __launch_bounds__(MAXT, MINB) sad_forward_kernel(SadArgs a) {
       const int xm = x - dv[q];
       r[q] = (xm >= 0 && xm < a.W) ? acc[p][q] : 40.0f;
     }
-    float* o = out + static_cast<int64_t>(x) * a.D + dg * kPD;
-    if ((a.D % 4 == 0) && dg * kPD + kPD <= a.D) {
+    float* o = out + static_cast<int64_t>(x) * a.D + a.g0 + dg * kPD;
+    if ((a.D % 4 == 0) && dg * kPD + kPD <= a.n) {
       reinterpret_cast<float4*>(o)[0] = make_float4(r[0], r[1], r[2], r[3]);
       reinterpret_cast<float4*>(o)[1] = make_float4(r[4], r[5], r[6], r[7]);
     } else {
 #pragma unroll
       for (int q = 0; q < kPD; ++q)
-        if (dg * kPD + q < a.D) o[q] = r[q];
+        if (dg * kPD + q < a.n) o[q] = r[q];
     }
   }
 }
@@ -659,38 +662,50 @@ extern "C" int bpl_sad_forward(const float* f0, const float* f1, float* out, int
   BPL_REQUIRE(step > 0.0f, "sad_forward: step must be > 0");
   const int D = bpl_sad_volume_depth(min_disp, max_disp, step);
   BPL_REQUIRE(D >= 1, "sad_forward: empty disparity range");
-  SadArgs a{f0, f1, out, B, C, H, W, D, min_disp, step, step == 1.0f ? 1 : 0, 0, 0};
-  int lo = 1 << 30, hi = -(1 << 30);
-  for (int di = 0; di < D; ++di) {
-    const int d = a.unit_step ? di + min_disp
-                              : static_cast<int>(static_cast<float>(di) * step + static_cast<float>(min_disp));
-    lo = std::min(lo, d);
-    hi = std::max(hi, d);
-  }
-  // for fractional steps the host's float rounding may differ from the
-  // device's by one: widen the staged span by one on each side
-  a.dlo = a.unit_step ? lo : lo - 1;
-  a.dhi = a.unit_step ? hi : hi + 1;
-  BPL_REQUIRE(a.dhi - a.dlo <= 4096, "sad_forward: disparity span %d too large", a.dhi - a.dlo);
-  const int ndg = (D + kPD - 1) / kPD;
-  const int threads = ndg * kPXG;
-  BPL_REQUIRE(threads <= 1024, "sad_forward: D=%d too large (at most %d disparities)", D, 1024 / (kTX / kPX) * kPD);
-  const int span = kTX + (a.dhi - a.dlo);
-  const int pad = a.unit_step ? sad_pad(a.dhi, a.dlo) : 0;
-  const size_t smem = 2 * sizeof(float) * kCChunk * (kTX + ((pad + span + 3) & ~3));  // two chunk buffers
-  BPL_REQUIRE(static_cast<int>(smem) <= max_smem_optin(), "sad_forward: disparity span too large");
-  auto launch = [&](auto kern) -> int {
-    if (smem > 48 * 1024)
-      BPL_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)),
-                   "cudaFuncSetAttribute");
-    dim3 grid((W + kTX - 1) / kTX, H, B);
-    kern<<<grid, threads, smem, as_stream(stream)>>>(a);
-    BPL_CUDA_TRY(cudaGetLastError(), "sad_forward launch");
-    return BPL_OK;
+  SadArgs a{f0, f1, out, B, C, H, W, D, 0, D, min_disp, step, step == 1.0f ? 1 : 0, 0, 0};
+  // the disparities [g0, g0 + n) as the launch of a; the bytes of its two chunk buffers
+  auto range = [&](int g0, int n) -> size_t {
+    int lo = 1 << 30, hi = -(1 << 30);
+    for (int di = g0; di < g0 + n; ++di) {
+      const int d = a.unit_step ? di + min_disp
+                                : static_cast<int>(static_cast<float>(di) * step + static_cast<float>(min_disp));
+      lo = std::min(lo, d);
+      hi = std::max(hi, d);
+    }
+    a.g0 = g0;
+    a.n = n;
+    // for fractional steps the host's float rounding may differ from the
+    // device's by one: widen the staged span by one on each side
+    a.dlo = a.unit_step ? lo : lo - 1;
+    a.dhi = a.unit_step ? hi : hi + 1;
+    const int span = kTX + (a.dhi - a.dlo);
+    const int pad = a.unit_step ? sad_pad(a.dhi, a.dlo) : 0;
+    return 2 * sizeof(float) * kCChunk * (kTX + ((pad + span + 3) & ~3));
   };
-  if (threads <= 256) return launch(sad_forward_kernel<256, 3>);
-  if (threads <= 384) return launch(sad_forward_kernel<384, 2>);
-  return launch(sad_forward_kernel<512, 1>);
+  BPL_REQUIRE(D <= 2 * kMaxD, "sad_forward: D=%d too large (at most %d disparities)", D, 2 * kMaxD);
+  const size_t whole = range(0, D);
+  BPL_REQUIRE(a.dhi - a.dlo <= 4096, "sad_forward: disparity span %d too large", a.dhi - a.dlo);
+  BPL_REQUIRE(static_cast<int>(whole) <= max_smem_optin(), "sad_forward: disparity span too large");
+  // above kMaxD disparities in two launches of about half
+  const int per = (D <= kMaxD) ? D : ((D + 1) / 2 + kPD - 1) / kPD * kPD;
+  for (int g0 = 0; g0 < D; g0 += per) {
+    const size_t smem = range(g0, std::min(per, D - g0));
+    const int threads = (a.n + kPD - 1) / kPD * kPXG;
+    auto launch = [&](auto kern) -> int {
+      if (smem > 48 * 1024)
+        BPL_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)),
+                     "cudaFuncSetAttribute");
+      dim3 grid((W + kTX - 1) / kTX, H, B);
+      kern<<<grid, threads, smem, as_stream(stream)>>>(a);
+      BPL_CUDA_TRY(cudaGetLastError(), "sad_forward launch");
+      return BPL_OK;
+    };
+    const int st = (threads <= 256)   ? launch(sad_forward_kernel<256, 3>)
+                   : (threads <= 384) ? launch(sad_forward_kernel<384, 2>)
+                                      : launch(sad_forward_kernel<512, 1>);
+    if (st != BPL_OK) return st;
+  }
+  return BPL_OK;
 }
 
 extern "C" int bpl_sad_backward(const float* f0, const float* f1, const float* in_grad, float* df0, float* df1,
