@@ -68,7 +68,11 @@ constexpr int kPXG = kTX / kPX;  // pixel groups per block
 // leading pad of an f1 row: (window start + pad) % 4 == 0 for every thread
 __host__ __device__ inline int sad_pad(int dhi, int dlo) { return ((7 - (dhi - dlo)) % 4 + 4) % 4; }
 
-// grid (ceil(W/kTX), H, B); block kPXG x (n/kPD rounded up) threads.
+// grid (ceil(W/kTX), H, B); block kPXG x (n/kPD rounded up) threads, rounded
+// up to whole warps: a half warp would stage its share of the rows in twice
+// the time, and the staging loops would need a run-time stride (376x1240,
+// C = 64: D = 192 727 -> 665 us, D = 24 257 -> 164 us; 333x145, C = 64, D = 22
+// at step 1/2 75 -> 65 us, 71 before rows went to warps).
 // MAXT/MINB: blocks of up to 384 threads run with registers capped (80, no
 // spills) so that 2-3 blocks stay resident per SM and one block's chunk
 // barrier does not idle the SM; 512-thread blocks (D > 192) keep theirs.
@@ -83,7 +87,6 @@ __global__ void __launch_bounds__(MAXT, MINB) sad_forward_kernel(SadArgs a) {
   const int xb = x0 - a.dhi - pad;             // f1 column of s1[.][0]
   const int ndg = (a.n + kPD - 1) / kPD;
   const int tid = threadIdx.x;
-  const int nthreads = blockDim.x;
   const int xg = tid % kPXG;                   // pixel group
   const int dg = tid / kPXG;                   // disparity group
   const bool active = dg < ndg;
@@ -100,8 +103,7 @@ __global__ void __launch_bounds__(MAXT, MINB) sad_forward_kernel(SadArgs a) {
 #pragma unroll
     for (int q = 0; q < kPD; ++q) acc[p][q] = 0.0f;
 
-  // (blocks are 16 threads per disparity group: the last warp may be half one)
-  const int lane = tid & 31, wl = min(32, nthreads - (tid & ~31));
+  const int lane = tid & 31;
   // staged f1 columns inside the image and the span
   const int lo = max(pad, -xb), hi = min(pad + span, a.W - xb);
   // stage chunk `ci` into buffer ci & 1 (cp.async; zeros outside the image)
@@ -112,17 +114,17 @@ __global__ void __launch_bounds__(MAXT, MINB) sad_forward_kernel(SadArgs a) {
     float* s1 = s0 + kCChunk * kTX;
     // one warp per channel row: no division per element (a run-time one for
     // each of the 5000 staged values took a quarter of the instructions)
-    const int nw = (nthreads + 31) >> 5;
+    const int nw = blockDim.x >> 5;
     for (int cc = tid >> 5; cc < cn; cc += nw) {
       const float* r0 = f0 + (c0 + cc) * HW + x0;
       const float* r1 = f1 + (c0 + cc) * HW + xb;
       float* d0 = s0 + cc * kTX;
       float* d1 = s1 + cc * spanp;
-      for (int xx = lane; xx < kTX; xx += wl) {
+      for (int xx = lane; xx < kTX; xx += 32) {
         if (xx < a.W - x0) cp_async4(d0 + xx, r0 + xx);
         else d0[xx] = 0.0f;
       }
-      for (int xx = lane; xx < spanp; xx += wl) {
+      for (int xx = lane; xx < spanp; xx += 32) {
         if (xx >= lo && xx < hi) cp_async4(d1 + xx, r1 + xx);
         else d1[xx] = 0.0f;
       }
@@ -690,7 +692,7 @@ extern "C" int bpl_sad_forward(const float* f0, const float* f1, float* out, int
   const int per = (D <= kMaxD) ? D : ((D + 1) / 2 + kPD - 1) / kPD * kPD;
   for (int g0 = 0; g0 < D; g0 += per) {
     const size_t smem = range(g0, std::min(per, D - g0));
-    const int threads = (a.n + kPD - 1) / kPD * kPXG;
+    const int threads = ((a.n + kPD - 1) / kPD * kPXG + 31) & ~31;
     auto launch = [&](auto kern) -> int {
       if (smem > 48 * 1024)
         BPL_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)),

@@ -1,4 +1,4 @@
-"""SAD volumes of more than 256 disparities, up to the 512 that the call
+"""SAD forward: volumes with an odd number of disparity groups, and of more than 256 disparities, up to the 512 that the call
 accepts (two launches), against the oracle: bit-exact, whole and fractional
 steps, ranges that start below zero, counts around the halves and their groups
 of eight."""
@@ -23,6 +23,20 @@ def test_more_than_256_disparities(C, H, W, lo, hi, step):
     dev = torch.device("cuda:0")
     vol = ops.sad_forward(torch.from_numpy(f0).to(dev), torch.from_numpy(f1).to(dev), lo, hi, step)
     np.testing.assert_array_equal(vol.cpu().numpy(), oracle.sad_forward(f0, f1, lo, hi, step))
+
+
+@pytest.mark.parametrize("D", [1, 8, 17, 24, 33, 40, 129, 250])
+@pytest.mark.parametrize("step", [1.0, 0.5])
+def test_odd_groups_of_disparities(D, step):
+    """Blocks whose last warp is half without disparities."""
+    from bpl_gb300 import ops
+    g = np.random.default_rng(D)
+    f0 = g.normal(size=(1, 21, 3, 150)).astype(np.float32)
+    f1 = g.normal(size=(1, 21, 3, 150)).astype(np.float32)
+    hi = int(D * step) - 1
+    dev = torch.device("cuda:0")
+    vol = ops.sad_forward(torch.from_numpy(f0).to(dev), torch.from_numpy(f1).to(dev), -1, hi, step)
+    np.testing.assert_array_equal(vol.cpu().numpy(), oracle.sad_forward(f0, f1, -1, hi, step))
 
 
 def test_513_disparities_are_refused():
