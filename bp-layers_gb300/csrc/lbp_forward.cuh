@@ -948,7 +948,7 @@ __global__ void __launch_bounds__(32 * fwd_block_warps<OCC>(), OCC) lbp_forward_
       int lcnt = 0, llab = 0;
 #pragma unroll
       for (int kk = 0; kk < KW; ++kk) {
-        const bool eq = lvalid(kk) && h[kk] == pm;  // (a row of NaNs: the minimum is that of no label)
+        const bool eq = h[kk] == pm;
         lcnt += eq ? 1 : 0;
         llab = eq ? c.t0 + lane + 32 * kk : llab;
       }
@@ -1146,9 +1146,9 @@ __global__ void __launch_bounds__(32 * fwd_block_warps<OCC>(), OCC) lbp_forward_
           }
       }
       // exact ties of the minimum: the reference tree picks the label (and,
-      // between -0 and +0, the value); so it does where no label has it, a
-      // row of NaNs
-      if (tot != 1) {
+      // between -0 and +0, the value); so it does in a row of NaNs, whose
+      // minimum is the +inf of lanes without a label, or NaN
+      if (tot > 1 || !(min_h < kInf)) {
         float tv[K];
         int tl[K];
 #pragma unroll

@@ -273,12 +273,12 @@ __global__ void __launch_bounds__(32 * f16_block_warps<OCC>(), OCC) lbp_forward_
     __syncwarp();  // h of the whole pixel is visible in hs
     issue(SL, i + (kRing ? DEPTH - 1 : 2));  // (ring: over the rows of step i - 1, which every lane is past)
     if (AM) {
-      // (label 0 where no label's h equals the minimum, a row of NaNs: the
-      // adjoint adds at this index, so it has to be a label)
+      // (in a row of NaNs the minimum is NaN, or the +inf of lanes without a
+      // label: the adjoint adds at this index, so it has to be a label)
       int ll = 0;
 #pragma unroll
-      for (int kk = 0; kk < K; ++kk) ll = (lvalid(kk) && h[kk] == pm) ? lab(kk) : ll;
-      argmin_h = __reduce_max_sync(FULL, ll);
+      for (int kk = 0; kk < K; ++kk) ll = (h[kk] == pm) ? lab(kk) : ll;
+      argmin_h = min(__reduce_max_sync(FULL, ll), L - 1);
     }
   };
   // stores the row relative to the minimum of h (the chain carries the
@@ -366,9 +366,11 @@ __global__ void __launch_bounds__(32 * f16_block_warps<OCC>(), OCC) lbp_forward_
         const float m = fmin3(nl, n0, nr);
         msg[kk] = fminf(m, msg_g);
         if (AM) {
-          // the own label, then the left one, then the right one (by equality
-          // with the minimum: a NaN term is none of them)
-          const int arg = (n0 == m) ? lab(kk) : (nl == m) ? lab(kk) - 1 : lab(kk) + 1;
+          // the own label, then the left one, then the right one (by
+          // equality with a minimum: a NaN term is none of them)
+          const float ml = fminf(nl, n0);
+          int arg = (n0 == ml) ? lab(kk) : lab(kk) - 1;
+          arg = (ml == m) ? arg : lab(kk) + 1;
           am[kk] = (m < msg_g) ? arg : argmin_h;
         }
       }
