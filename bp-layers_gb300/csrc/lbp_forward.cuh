@@ -84,7 +84,6 @@ struct FwdArgs {
   int Ls;     // label stride of cost / messages / argmin rows
   int Lm;     // row stride of the pixel-pairwise matrices (pixel variant)
   int argmin_kind;
-  int half_align;  // half storage: cost and messages start on 16-byte boundaries
   int am_vec;  // uint8 argmin rows start on multiples of this many bytes and are multiples of it long (16, 4 or 1)
   int phase;  // 0: RIGHT+LEFT over rows, 1: DOWN+UP over columns
   int nchains;
@@ -98,6 +97,7 @@ struct FwdArgs {
   // transposed, DU the UD matrix of the pixel above, transposed
   // (message_passing_op_pw_pixel.py:27-38)
   int planes2;
+  int half_align;  // half storage: cost and messages start on 16-byte boundaries
 };
 
 // exp/log of the message normalisation with the reference's results
@@ -1070,29 +1070,82 @@ __global__ void __launch_bounds__(32 * fwd_block_warps<OCC>(), OCC) lbp_forward_
       if (!__all_sync(FULL, eok0) && !eok0) e[0] = static_cast<float>(exp(static_cast<double>(msg[0])));
     } else if (delta >= L) {
       // full minimisation (lbp_min_sum_kernel.cu:88-111): last minimiser wins
+      if constexpr (VARIANT == BPL_LBP_STEREO || kPixGlobal) {
 #pragma unroll
-      for (int kk = 0; kk < KW; ++kk) {
-        const int t = c.t0 + lane + 32 * kk;
-        float m = 1e15f;
-        int arg = 0;
-        if (t < L) {
-          for (int s = 0; s < L; ++s) {
-            float f;
-            if (stereo) {
-              const int ti = max(1, min(a.Lv - 1, a.Lv / 2 + (t - s)));
-              f = tile[ti * 33 + j];
-            } else if (VARIANT == BPL_LBP_SEM_GLOBAL) {
-              f = __ldg(gjump + s * L + t);
-            } else {
-              f = pairf(s, t);
+        for (int kk = 0; kk < KW; ++kk) {
+          const int t = c.t0 + lane + 32 * kk;
+          float m = 1e15f;
+          int arg = 0;
+          if (t < L) {
+            for (int s = 0; s < L; ++s) {
+              float f;
+              if constexpr (kPixGlobal) f = pairf(s, t);
+              else f = tile[max(1, min(a.Lv - 1, a.Lv / 2 + (t - s))) * 33 + j];
+              const float nm = __fmaf_rn(f, w, cs.hs[s]);
+              m = fminf(m, nm);
+              if (m == nm) arg = s;
             }
-            const float nm = __fmaf_rn(f, w, cs.hs[s]);
-            m = fminf(m, nm);
-            if (m == nm) arg = s;
+          }
+          msg[kk] = m;
+          am[kk] = arg;
+        }
+      } else {
+        // the slots side by side: one read of h per sender, and KW chains of
+        // minima in flight instead of one (lanes past L follow label L-1).
+        // One slot after the other this loop was 4 to 27 % slower than the
+        // one before it, by how it happened to be compiled (1x128x256: global
+        // L = 64 1.25 ms, L = 128 5.41, pixel L = 64 1.95; 1.13, 4.77, 1.53
+        // before); now 1.09, 4.17 and 1.53 ms.
+#pragma unroll
+        for (int kk = 0; kk < KW; ++kk) {
+          msg[kk] = 1e15f;
+          am[kk] = 0;
+        }
+        auto entry = [&](int s, int kk) -> float {
+          const int t = min(c.t0 + lane + 32 * kk, L - 1);
+          if constexpr (VARIANT == BPL_LBP_SEM_GLOBAL) return __ldg(gjump + s * L + t);
+          else return pairf(s, t);
+        };
+        auto take = [&](int s, int kk, float f, float hv) {
+          const float nm = __fmaf_rn(f, w, hv);
+          msg[kk] = fminf(msg[kk], nm);
+          if (msg[kk] == nm) am[kk] = s;
+        };
+        int s = 0;
+        if constexpr (kRing && KW == 2) {
+          // senders in groups of four, their h by one read: the matrices are
+          // in shared memory too, whose reads bound the loop (1.66 ms without;
+          // at three slots, and from global memory, it is the slower form)
+#pragma unroll 2
+          for (; s + 4 <= L; s += 4) {
+            const float4 h4 = *reinterpret_cast<const float4*>(cs.hs + s);
+            float f[4][KW];
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+#pragma unroll
+              for (int kk = 0; kk < KW; ++kk) f[q][kk] = entry(s + q, kk);
+#pragma unroll
+            for (int kk = 0; kk < KW; ++kk) {
+              take(s, kk, f[0][kk], h4.x);
+              take(s + 1, kk, f[1][kk], h4.y);
+              take(s + 2, kk, f[2][kk], h4.z);
+              take(s + 3, kk, f[3][kk], h4.w);
+            }
           }
         }
-        msg[kk] = m;
-        am[kk] = arg;
+#pragma unroll(KW <= 2 ? 4 : KW <= 4 ? 2 : 1)
+        for (; s < L; ++s) {
+          const float hv = cs.hs[s];
+#pragma unroll
+          for (int kk = 0; kk < KW; ++kk) take(s, kk, entry(s, kk), hv);
+        }
+#pragma unroll
+        for (int kk = 0; kk < KW; ++kk) {
+          if (!lvalid(kk)) {
+            msg[kk] = 1e15f;
+            am[kk] = 0;
+          }
+        }
       }
       bool all_ok = true;
       bool eok[KW];
