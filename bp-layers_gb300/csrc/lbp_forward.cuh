@@ -711,6 +711,15 @@ __global__ void __launch_bounds__(32 * fwd_block_warps<OCC>(), OCC) lbp_forward_
     }
     __syncwarp();
   };
+  // kLean: this lane's line (of K + 1 per row) of the three rows, for the L2
+  // prefetch of the hot loop
+  constexpr bool kAhead = OCC == 1 || (PH == 1 && K <= 4);
+  const char* pf_row = nullptr;
+  if constexpr (kLean && kAhead) {
+    const int prow = lane / (K + 1), pline = lane % (K + 1);
+    pf_row = reinterpret_cast<const char*>(prow == 1 ? c.slot_a : prow == 2 ? c.slot_b : c.cost) +
+             ((prow < 3 && 32 * pline < L) ? 128 * pline : 0);
+  }
   for (int i = 0; i < nsteps; ++i, pin += c.dpin) {
     float h[KW], pm;
     float msg[KW];
@@ -727,10 +736,19 @@ __global__ void __launch_bounds__(32 * fwd_block_warps<OCC>(), OCC) lbp_forward_
       // second sender within rounding of the candidate, a window term equal
       // to the candidate or to 0 (ties and their signs), several labels
       // below the candidate in a lane or one in every lane, a rounding of
-      // exp or log that is undecided, an infinite minimum or candidate, or a
-      // record of another form; that step runs the code after the loop, which
-      // is kept out of the hot loop's way.  (A NaN term is dropped here as by
-      // the forms there: no minimum and no vote sees it.)  WIDE: taps at distance 2 below L2.
+      // exp or log that is undecided, or an infinite minimum or candidate;
+      // that step runs the code after the loop, which is kept out of the hot
+      // loop's way.  A step whose record is of another form leaves as soon as
+      // it has its h.  (A NaN term is dropped here as by the forms there: no
+      // minimum and no vote sees it.)  WIDE: taps at distance 2 below L2.
+      // A step outside the loop costs its block, or the part before the form
+      // test, and the way back in.  With the form in the vote, after the whole
+      // block, scanlines of weights <= 0, offsets or windows beyond kFastDelta
+      // took up to 1.24 times as long as before there was a loop (188x620x96,
+      // all weights 0: 1.20 ms, 0.99 before, 0.99 now; two passes with offsets
+      // 4.38 / 3.81 / 3.79).  A loop of its own for such steps takes a third of
+      // that off again, but its registers and code cost the others 1 to 20 %; a
+      // second place for the h and the loads waited for the loads.
       // (Moving the stores and the next step's h before the vote, to overlap
       // it, gained 2 % on the latency-bound launch and lost 3 % on the
       // others.)
@@ -756,12 +774,7 @@ __global__ void __launch_bounds__(32 * fwd_block_warps<OCC>(), OCC) lbp_forward_
         // vertical launch at 4x256x512x96 0.43 -> 0.35 ms).  At 192 labels
         // the vertical launch already streams at 80 % of the copy rate and
         // it costs 5 %; along rows with 13 warps per SM it costs 4 %.
-        constexpr bool kAhead = OCC == 1 || (PH == 1 && K <= 4);
-        const int prow = lane / (K + 1), pline = lane % (K + 1);
-        const bool pf_lane = prow < 3 && 32 * pline < L;
-        const char* ppf = reinterpret_cast<const char*>((prow == 1 ? c.slot_a : prow == 2 ? c.slot_b : c.cost) +
-                                                        (static_cast<int64_t>(pin) + min(kL2Ahead, nsteps - 1 - i) * c.dpin) * Ls) +
-                          (pf_lane ? 128 * pline : 0);
+        const char* ppf = pf_row + (static_cast<int64_t>(pin) + min(kL2Ahead, nsteps - 1 - i) * c.dpin) * Ls * sizeof(T);
         for (;;) {
           const float4 lt = *rec;
           const float w = kWide ? -lt.x : lt.x;
@@ -782,6 +795,9 @@ __global__ void __launch_bounds__(32 * fwd_block_warps<OCC>(), OCC) lbp_forward_
             prefetch_l2(ppf);
             ppf += (i + kL2Ahead + 1 < nsteps) ? pstep * static_cast<int64_t>(sizeof(T)) : 0;
           }
+          // a record of another form: the step has its h and its next rows on
+          // their way, and leaves before the block
+          if (!(w > 0.0f)) return;
           float mw[KW];
 #pragma unroll
           for (int kk = 0; kk < KW; ++kk) {
@@ -833,15 +849,14 @@ __global__ void __launch_bounds__(32 * fwd_block_warps<OCC>(), OCC) lbp_forward_
           if constexpr (kWide) arg = (arg == t || __fmaf_rn(lt.z, w, cs.hs[t - 1]) == xs) ? arg : t - 2;
           arg = (__fmaf_rn(lt.w, w, cs.hs[t + 1]) == xs) ? t + 1 : arg;
           if constexpr (kWide) arg = (__fmaf_rn(l2.y, w, cs.hs[t + 2]) == xs) ? t + 2 : arg;
-          const bool form = w > 0.0f;
           const bool near1 = near < 0x20000 && (nearl & (nearl - 1u)) == 0u && nearl != 0u;
           const float sum = tree_sum<K>(ev);
           float lse;
           const bool okl = crm::log_fast(sum, lse, s_log);
-          const bool good = form && near1 && own < 0x20000 && ownl != FULL && okx && okl &&
+          const bool good = near1 && own < 0x20000 && ownl != FULL && okx && okl &&
                             (own == 0 || (xs != msg_g && xs != 0.0f));
           if (!__all_sync(FULL, good)) {
-            lean_dense = __all_sync(FULL, form && near1);
+            lean_dense = __all_sync(FULL, near1);
             return;
           }
 #pragma unroll
