@@ -36,25 +36,104 @@ template <int OCC>
 constexpr int f16_depth = (OCC > 1) ? 0 : 8;
 // steps ahead of the L2 prefetch (no ring)
 constexpr int kF16Ahead = 8;
-// floats of a warp's shared memory: h row, ring, two tap tiles
+// floats of a warp's shared memory: h row, ring, two tap tiles, and the rows
+// of messages and index bytes that f16_any_window leaves
 __host__ __device__ inline int f16_warp_floats(int NP, int depth, int Lv) {
-  return align4(64 * NP + 2 * kHsPad) + depth * 3 * 32 * NP + 2 * tap_tile_floats(Lv, true);
+  return align4(64 * NP + 2 * kHsPad) + depth * 3 * 32 * NP + 2 * tap_tile_floats(Lv, true) + 80 * NP;
 }
 
 template <int OCC>
 constexpr int f16_block_warps() { return (OCC > 1) ? 1 : 4; }
 
-// The window of a sender as the usual step reads it: {w, L2, f(t-1), f(t+1)}
-// and {f(t), 1 where the beating offsets are exactly |jd| <= 1 (see
-// classify_taps), else 0}, in the place of the float kernel's lean records.
+// The window of a sender as a step reads it: {w, L2, f(t-1), f(t+1)} and
+// {f(t), form}, in the place of the float kernel's lean records.  Form 1, the
+// usual window: the beating offsets are exactly |jd| <= 1 (see classify_taps);
+// 2: no offset beyond |jd| = 2 beats; 0: any other window.  A tap that does
+// not beat gives the candidate's value or more everywhere, so a window of form
+// 2 is its five inner terms, whether these beat or not (learned affinities,
+// where a tap at one side often equals L2, and any window wider than the taps;
+// two passes at 188x620x96 with affinities 2.52 -> 1.03 ms with such steps in
+// pairs, 2.11 before labels went to pairs; a window of 7 3.39 -> 1.01, 2.79
+// before).
 __device__ __forceinline__ void store_f16_record(const FwdArgs& a, float* tile, int lane) {
   const int c0 = a.Lv / 2;
   const int code = __float_as_int(tile[(a.Lv + 2) * 33 + lane]) & 0xff;
+  const float w = tile[a.Lv * 33 + lane], L2 = tile[(a.Lv - 1) * 33 + lane];
+  bool near = tile[lane] == 0.0f && a.delta >= 2 && a.delta < a.L;
+  // (offsets beyond the taps' own all read the same two)
+  for (int q = 3; q <= min(a.delta, max(3, c0)); ++q) {
+    const float fp = tile[max(1, c0 - q) * 33 + lane], fm = tile[min(a.Lv - 1, c0 + q) * 33 + lane];
+    const float lo = (w >= 0.0f) ? fminf(fp, fm) : fmaxf(fp, fm);
+    near = near && fp == fp && fm == fm && (w > 0.0f ? lo >= L2 : w < 0.0f ? lo <= L2 : w == 0.0f);
+  }
+  const float form = (code == 3 && a.delta < a.L) ? 1.0f : near ? 2.0f : 0.0f;
   float* rec = tile + lean_off(a.Lv);
   reinterpret_cast<float4*>(rec)[lane] =
-      make_float4(tile[a.Lv * 33 + lane], tile[(a.Lv - 1) * 33 + lane], tile[min(a.Lv - 1, c0 + 1) * 33 + lane],
-                  tile[max(1, c0 - 1) * 33 + lane]);
-  reinterpret_cast<float2*>(rec + 128)[lane] = make_float2(tile[c0 * 33 + lane], code == 3 ? 1.0f : 0.0f);
+      make_float4(w, L2, tile[min(a.Lv - 1, c0 + 1) * 33 + lane], tile[max(1, c0 - 1) * 33 + lane]);
+  reinterpret_cast<float2*>(rec + 128)[lane] = make_float2(tile[c0 * 33 + lane], form);
+}
+
+// A step of any window: the full minimisation (delta >= L,
+// lbp_min_sum_kernel.cu:88-111) or the reference's rounded start / stop around
+// t + offset (:112-164).  taps: column j of the sender's tile, hs: the row of
+// h; messages go to out[0 .. L-1], indices (L <= 256) to the bytes 32 K floats
+// further on.  Label lane + 32 k, so that few labels fill the lanes and the reads
+// of h meet no bank conflicts (in pairs these loops took up to 1.85 times as
+// long), one slot at a time and through shared memory, so that the usual
+// step's registers and code stay as they are (two passes at 188x620x96 with
+// offsets 2.72 -> 1.97 ms, 2.25 before labels went to pairs; the full
+// minimisation, 1x188x310, L = 32, 0.64 -> 0.53 ms, 0.35 before).
+template <int K>
+__device__ __forceinline__ void f16_any_window(const float* hs, const float* taps, float* out, int L, int Lv, int delta,
+                                               float w, float msg_g, int argmin_h) {
+  uint8_t* idx = reinterpret_cast<uint8_t*>(out + 32 * K);
+  const int c0 = Lv / 2, lane = threadIdx.x & 31;
+  const float kInf = __int_as_float(0x7f800000);
+  const bool full = delta >= L;
+  const float off = taps[0];
+#pragma unroll 1
+  for (int t = lane; t < L; t += 32) {
+    float m = kInf;
+    int arg = 0;
+    // senders start .. stop - 1, eight at a time (their loads and products in
+    // flight together, and one comparison with the minimum so far); among equal
+    // ones the last (LAST) or the first wins
+    auto scan = [&](auto LAST, int start, int stop) {
+      constexpr bool kLast = decltype(LAST)::value;
+#pragma unroll 1
+      for (int s = start; s < stop; s += 8) {
+        float n[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          // (past stop: inside the warp's shared memory, and not used; h is
+          // +inf past L, where the full minimisation stops)
+          const float v = __fmaf_rn(taps[max(1, min(Lv - 1, c0 + (t - s - q))) * 33], w, hs[s + q]);
+          n[q] = (kLast || s + q < stop) ? v : kInf;
+        }
+        const float b = min_of<8>(n);
+        if (kLast ? b <= m : b < m) {
+          m = b;
+#pragma unroll
+          for (int r = 0; r < 8; ++r) {
+            const int q = kLast ? r : 7 - r;
+            arg = (n[q] == b) ? s + q : arg;
+          }
+        }
+      }
+    };
+    if (full) {
+      scan(std::true_type{}, 0, L);
+      out[t] = m;
+      idx[t] = static_cast<uint8_t>(min(arg, L - 1));
+      continue;
+    }
+    scan(std::false_type{},
+         sat_u16(roundf(__fsub_rn(__fadd_rn(static_cast<float>(t - (delta - 1)), off), 1.0f))),
+         min(sat_u16(roundf(__fadd_rn(__fadd_rn(static_cast<float>(t + delta), off), 1.0f))), L));
+    const bool win = m < msg_g;
+    out[t] = win ? m : msg_g;
+    idx[t] = static_cast<uint8_t>(win ? arg : argmin_h);
+  }
 }
 
 // Labels in pairs: lane l holds labels 64 p + 2 l and the next one, p < NP =
@@ -99,6 +178,7 @@ __global__ void __launch_bounds__(32 * f16_block_warps<OCC>(), OCC) lbp_forward_
   float* hs = base + kHsPad;
   __half* ring = reinterpret_cast<__half*>(base + align4(32 * K + 2 * kHsPad));  // [DEPTH][3][64 NP]
   float* taps = base + align4(32 * K + 2 * kHsPad) + DEPTH * 3 * 32 * NP;
+  float* rows_out = taps + 2 * tile_stride;  // [64 NP] messages, [64 NP] index bytes (f16_any_window)
   if (lane < kHsPad) {
     hs[-1 - lane] = __int_as_float(0x7f800000);
     hs[32 * K + lane] = __int_as_float(0x7f800000);
@@ -343,18 +423,18 @@ __global__ void __launch_bounds__(32 * f16_block_warps<OCC>(), OCC) lbp_forward_
     }
     return i == nsteps;
   };
-  // One step of the usual window (lbp_min_sum_kernel.cu:112-164 with the
-  // terms |jd| <= 1): the candidate L2*w + min h, and the terms that can beat
-  // it.  0: done, 1: the general step has to finish it, 2: end of the
+  // One step of the usual window (lbp_min_sum_kernel.cu:112-164 with the terms
+  // |jd| <= 1): the candidate L2*w + min h, and the terms that can beat
+  // it.  0: done, 1: another window, to be finished below, 2: end of the
   // scanline.
   auto usual = [&](auto SL) -> int {
     const float* rec = taps + ((i >> 5) & 1) * tile_stride + lean_off(a.Lv);
     const float4 lt = reinterpret_cast<const float4*>(rec)[i & 31];
     const float2 l2 = reinterpret_cast<const float2*>(rec + 128)[i & 31];
     head(SL);
-    if (l2.y == 0.0f || delta >= L) return 1;
     const float w = lt.x;
     const float msg_g = __fmaf_rn(lt.y, w, pm);
+    if (__builtin_expect(l2.y != 1.0f, 0)) return 1;
 #pragma unroll
     for (int p = 0; p < NP; ++p) {
       const float hl = hs[64 * p + 2 * lane - 1], hr = hs[64 * p + 2 * lane + 2];
@@ -377,7 +457,6 @@ __global__ void __launch_bounds__(32 * f16_block_warps<OCC>(), OCC) lbp_forward_
     }
     return tail() ? 2 : 0;
   };
-  // (the general step is kept out of the loop's way)
   auto run = [&]() -> int {
     for (;;) {
       if constexpr (kRing) {
@@ -389,70 +468,48 @@ __global__ void __launch_bounds__(32 * f16_block_warps<OCC>(), OCC) lbp_forward_
       }
     }
   };
+  // (the other windows are kept out of the loop's way)
   while (run() == 1) {
-    const int j = i & 31;
-    const float* tile = taps + ((i >> 5) & 1) * tile_stride;
-    const float w = tile[a.Lv * 33 + j];
-    if (delta >= L) {
-      // full minimisation (lbp_min_sum_kernel.cu:88-111)
+    const float* tile = taps + ((i >> 5) & 1) * tile_stride + (i & 31);
+    const float w = tile[a.Lv * 33];
+    const float msg_g = __fmaf_rn(tile[(a.Lv - 1) * 33], w, pm);
+    if (reinterpret_cast<const float2*>(taps + ((i >> 5) & 1) * tile_stride + lean_off(a.Lv) + 128)[i & 31].y == 2.0f) {
+      // senders t-2 .. t+2, the first minimiser wins
+      float f[5];
 #pragma unroll
-      for (int kk = 0; kk < K; ++kk) {
-        const int t = lab(kk);
-        float m = kInf;
-        int arg = 0;
-        if (t < L) {
-          for (int s = 0; s < L; ++s) {
-            const float f = tile[max(1, min(a.Lv - 1, c0 + (t - s))) * 33 + j];
-            const float nm = __fmaf_rn(f, w, hs[s]);
-            if (nm <= m) {
-              m = nm;
-              arg = s;
-            }
+      for (int q = 0; q < 5; ++q) f[q] = tile[max(1, min(a.Lv - 1, c0 + 2 - q)) * 33];
+#pragma unroll
+      for (int p = 0; p < NP; ++p) {
+        const float2 lo = *reinterpret_cast<const float2*>(hs + 64 * p + 2 * lane - 2);
+        const float2 hi = *reinterpret_cast<const float2*>(hs + 64 * p + 2 * lane + 2);
+        const float x[6] = {lo.x, lo.y, h[2 * p], h[2 * p + 1], hi.x, hi.y};
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          const int kk = 2 * p + k;
+          float n[5];
+#pragma unroll
+          for (int q = 0; q < 5; ++q) n[q] = __fmaf_rn(f[q], w, x[q + k]);
+          const float m = fmin3(fmin3(n[0], n[1], n[2]), n[3], n[4]);
+          msg[kk] = fminf(m, msg_g);
+          if (AM) {
+            int arg = lab(kk) + 2;
+#pragma unroll
+            for (int q = 3; q >= 0; --q) arg = (n[q] == m) ? lab(kk) + q - 2 : arg;
+            am[kk] = (m < msg_g) ? arg : argmin_h;
           }
         }
-        msg[kk] = m;
-        am[kk] = arg;
       }
     } else {
-      const float msg_g = __fmaf_rn(tile[(a.Lv - 1) * 33 + j], w, pm);
-      const int wcode = __float_as_int(tile[(a.Lv + 2) * 33 + j]);
-      const int R = ((wcode & 0xff) != kWinGeneric) ? (wcode & 0xff) - 2 : -2;
-      const float off = tile[0 * 33 + j];
-      float fR[5];
+      f16_any_window<K>(hs, tile, rows_out, L, a.Lv, delta, w, msg_g, argmin_h);
+      __syncwarp();
 #pragma unroll
-      for (int q = 0; q < 5; ++q) fR[q] = tile[max(1, min(a.Lv - 1, c0 - (q - 2))) * 33 + j];
-#pragma unroll
-      for (int kk = 0; kk < K; ++kk) {
-        const int t = lab(kk);
-        float m = kInf;
-        int arg = 0;
-        if (R >= -1) {
-          // R in {-1, 0, 2}: taps of senders t-2 .. t+2 (terms beyond R skipped)
-#pragma unroll
-          for (int q = 0; q < 5; ++q) {
-            const int jd = q - 2;
-            const float nm = __fmaf_rn(fR[q], w, hs[t + jd]);
-            const bool take = (jd >= -R) && (jd <= R) && (nm < m);
-            m = take ? nm : m;
-            arg = take ? t + jd : arg;
-          }
-        } else if (t < L) {
-          // generic window (offsets, wider beating ranges): the reference's
-          // rounded start / stop around t + offset
-          const int start = sat_u16(roundf(__fsub_rn(__fadd_rn(static_cast<float>(t - (delta - 1)), off), 1.0f)));
-          const int stop = min(sat_u16(roundf(__fadd_rn(__fadd_rn(static_cast<float>(t + delta), off), 1.0f))), L);
-          for (int s = start; s < stop; ++s) {
-            const float f = tile[max(1, min(a.Lv - 1, c0 + (t - s))) * 33 + j];
-            const float nm = __fmaf_rn(f, w, hs[s]);
-            if (nm < m) {
-              m = nm;
-              arg = s;
-            }
-          }
-        }
-        const bool win = m < msg_g;
-        msg[kk] = win ? m : msg_g;
-        am[kk] = win ? arg : argmin_h;
+      for (int p = 0; p < NP; ++p) {  // (what lies past L is never stored)
+        const float2 v = *reinterpret_cast<const float2*>(rows_out + 64 * p + 2 * lane);
+        const uint16_t g = reinterpret_cast<const uint16_t*>(rows_out + 64 * NP)[32 * p + lane];
+        msg[2 * p] = v.x;
+        msg[2 * p + 1] = v.y;
+        am[2 * p] = g & 0xff;
+        am[2 * p + 1] = g >> 8;
       }
     }
     if (tail()) break;
