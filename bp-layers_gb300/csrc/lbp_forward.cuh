@@ -573,11 +573,13 @@ __global__ void __launch_bounds__(32 * fwd_block_warps<OCC>(), OCC) lbp_forward_
   const float* gjump =
       (VARIANT == BPL_LBP_SEM_GLOBAL) ? static_cast<const float*>(a.jump) + static_cast<int64_t>(c.dir) * L * L : nullptr;
   const bool stereo = (VARIANT == BPL_LBP_STEREO);
-  // Global pairwise with one label per lane (L <= 32): the lane's column of
-  // the direction's matrix, P[s][t] for its label t, held in registers for
-  // the whole scanline, so the full minimisation is L register FMAs against
-  // broadcast reads of h instead of L global (L1) loads per step.
-  constexpr bool kPcolRegs = (VARIANT == BPL_LBP_SEM_GLOBAL) && K == 1 && NW == 1;
+  // Global pairwise with one label per lane (L <= 32), half storage: the lane's
+  // column of the direction's matrix, P[s][t] for its label t, held in
+  // registers for the whole scanline, so the full minimisation is L register
+  // FMAs against broadcast reads of h instead of L global (L1) loads per step.
+  constexpr bool kPcolRegs = (VARIANT == BPL_LBP_SEM_GLOBAL) && K == 1 && NW == 1 && sizeof(T) == 2;
+  // (float storage up to 32 labels: lbp_forward_sem_full.cuh takes it)
+  constexpr bool kFullElsewhere = (VARIANT != BPL_LBP_STEREO) && K == 1 && sizeof(T) == 4;
   float pcol[kPcolRegs ? 32 : 1];
   if constexpr (kPcolRegs) {
 #pragma unroll
@@ -1083,7 +1085,7 @@ __global__ void __launch_bounds__(32 * fwd_block_warps<OCC>(), OCC) lbp_forward_
         eok0 = true;
       }
       if (!__all_sync(FULL, eok0) && !eok0) e[0] = static_cast<float>(exp(static_cast<double>(msg[0])));
-    } else if (delta >= L) {
+    } else if (!kFullElsewhere && delta >= L) {
       // full minimisation (lbp_min_sum_kernel.cu:88-111): last minimiser wins
       if constexpr (VARIANT == BPL_LBP_STEREO || kPixGlobal) {
 #pragma unroll
