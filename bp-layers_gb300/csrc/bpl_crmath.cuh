@@ -5,8 +5,9 @@
 // precision and rounded to float (ops/lbp_stereo/src/lbp_min_sum_kernel.cu:167,
 // :180-181).  GB300's FP64 rate is a small fraction of its FP32 rate, so
 // evaluating one double exp per message label makes the kernel FP64-bound.
-// Here exp(x) and log(s) are evaluated in float-float arithmetic (about 2^-44
-// relative error) with table-driven argument reduction after
+// Here exp(x) and log(s) are evaluated in float-float arithmetic (errors below
+// 2^-39 relative and 2^-36 + 2^-43 |e| absolute, e the exponent of s) with
+// table-driven argument reduction after
 //   P. T. P. Tang, "Table-driven implementation of the exponential function
 //   in IEEE floating-point arithmetic", ACM TOMS 15(2), 1989, and
 //   P. T. P. Tang, "Table-driven implementation of the logarithm function in

@@ -27,9 +27,12 @@
 //     (376x1240x192: 752 warps on 608 SM sub-partitions; about 430
 //     instructions and 1300 cycles a step where the general step takes 770
 //     and 2900), down columns DRAM (1.1 GB read per direction and 0.45
-//     written, 80 % of the copy rate).  A forward pass at 376x1240x192 went
-//     from 2.48 to 1.38 ms (rows 1.50 -> 0.83, columns 0.98 -> 0.55), at
-//     188x620x96 from 0.82 to 0.42 ms, at 4x256x512x96 from 1.34 to 0.79 ms.
+//     written, 80 % of the copy rate).  The time depends on the data: a step
+//     leaves the loop for ties with the candidate and for several labels below
+//     it in one lane.  A forward pass at 376x1240x192 went from 2.48 to 1.38 ms
+//     on random costs with L2 = 0.5 (rows 1.50 -> 0.83, columns 0.98 -> 0.55)
+//     and is 1.55 ms on the piecewise planar scene of the training step; random
+//     costs at 188x620x96 0.82 -> 0.42 ms, at 4x256x512x96 1.34 -> 0.79 ms.
 //   * Labels are spread over lanes (label = lane + 32k).  min/argmin and the
 //     exp-sum reproduce the reference's reduction tree (bpl_device.cuh); the
 //     exp/log of the normalisation are correctly rounded float evaluations
@@ -789,9 +792,8 @@ __global__ void __launch_bounds__(32 * fwd_block_warps<OCC>(), OCC) lbp_forward_
           }
           pm = warp_min_f32(slot_min<KW>(h));
           __syncwarp();
-          // (a branch of its own: loads in the block itself are moved down
-          // towards their use, and their latency with them; horizontal
-          // launch at 376x1240x192 0.99 ms without it)
+          // (a branch of its own: horizontal launch at 376x1240x192 0.99 ms
+          // with the loads in the block itself)
           if (i + 1 < nsteps) prefetch(i + 1);
           if (kAhead) {
             prefetch_l2(ppf);

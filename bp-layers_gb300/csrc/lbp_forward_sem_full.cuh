@@ -217,8 +217,7 @@ __global__ void __launch_bounds__(32, kSemBlocks) lbp_forward_sem_full_kernel(Fw
                                : __fadd_rn(__fadd_rn(__fadd_rn(nc, na), nb), chain);
     hs[lane] = valid ? hv : kInf;
     __syncwarp();
-    // (a branch of its own: loads in the block itself are moved down to their
-    // use)
+    // (a branch of its own, as in the stereo kernel's hot loop)
     if (i + 1 < nsteps) {
       pc += pstep;
       pa += pstep;

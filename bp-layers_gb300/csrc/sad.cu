@@ -254,8 +254,7 @@ __device__ __forceinline__ void cp_async_or_zero(void* dst, const void* src, boo
 // df1 -= (diff/|diff|) g when |diff| > 1e-15.  diff/|diff| is exactly +-1 and
 // its product with g exact, so each update rounds once, like the
 // reference's; a NaN diff never passes the test.
-// (Written in PTX so that both updates are predicated: the compiler's form of
-// the same statements had seven instructions.)
+// (Written in PTX so that both updates are predicated.)
 __device__ __forceinline__ void sad_pair(float v0, float v1, float g, float& a0, float& a1) {
   asm("{\n"
       " .reg .f32 d, e, s, t;\n .reg .b32 u;\n .reg .pred p;\n"
@@ -512,7 +511,7 @@ __device__ __forceinline__ void sad_term(float& acc, float diff, float g) {
 }
 
 // Both gradients gathered per pixel, for problems with too few rows for the
-// strips below to fill the SMs (sad_bwd_gather).
+// strips above to fill the SMs (sad_bwd_gather).
 // grid (ceil(W/32), H, B*ceil(C/32)); block 256 = 8 warps.  Warp w owns
 // pixels x0 + 4w .. +3, lane the channel; both sums run over d ascending
 // (the reference's order), chunk by chunk of 32 disparities staged in
